@@ -12,7 +12,13 @@ namespace detail {
 constexpr int RUN = 4;
 constexpr int BPR_WARPS = 4;
 constexpr int BPR_CHUNK = 32;
-constexpr int BPR_LIST = 1024;  // class angles listed per window of the angle axis
+// Class angles listed per window of the angle axis.  The lists and tables of
+// the resident blocks come out of the SM's unified storage, and what they
+// leave is the L1 that the windows' reuse lives in: with 1024 (4 KB of list per
+// warp, 186 KB per SM in the 4-height form) A^T took 118 us at 128^3 and 192
+// angles and 70 us at 64^3 and 128, with 256 101 and 35 us (512^3: 4.36 and
+// 4.33 ms; 128 measured as 256).
+constexpr int BPR_LIST = 256;
 constexpr int BPR_GENERIC = 8;  // pattern value of the generic path
 constexpr int BPR_SKIP = 9;     // pattern value of a window wholly off the detector
 
