@@ -163,7 +163,9 @@ __global__ void __launch_bounds__(32 * BPB_WARPS)
 // PDL: the launch follows another run launch of the same call
 // programmatically (launch_ex), so its warps wait for that launch before they
 // add into x; a call's first launch keeps the form without the wait.
-template <int PASS, int R, bool ADD = false, bool FULL = false, bool PDL = false>
+// VOUT: see bp_runs_warp.
+template <int PASS, int R, bool ADD = false, bool FULL = false, bool PDL = false,
+          bool VOUT = true>
 __global__ void __launch_bounds__(32 * BPR_WARPS, R == 8 ? 5 : 0)
     bp_z0_runs_kernel(const float* __restrict__ y, float* __restrict__ x,
                       const float* __restrict__ angles, Geom g, int nrun_major, int run_base,
@@ -188,7 +190,7 @@ __global__ void __launch_bounds__(32 * BPR_WARPS, R == 8 ? 5 : 0)
   run_origin<PASS>(run, nrun_major, &xi0, &yi0);
   if (yi0 >= row_end) return;
   using Wait = std::conditional_t<PDL, PdlWait, NoWait>;
-  bp_runs_warp<PASS, R, Wait, ADD, FULL>(y, x, angles, g, xi0, yi0,
+  bp_runs_warp<PASS, R, Wait, ADD, FULL, VOUT>(y, x, angles, g, xi0, yi0,
                                          blockIdx.y * 32 * R + lane * 4, accumulate, tab[w],
                                          alist[w], Wait(), addend);
 }
@@ -432,6 +434,25 @@ cudaError_t launch_bp_z0_runs_tma(const float* y, float* x, const float* angles,
   return cudaSuccess;
 }
 
+// Rows of y take float4 loads; rows of x float4 stores.
+bool bp0_vec_in(const float* y, const Geom& g) {
+  return g.Hy % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+}
+bool bp0_vec_out(const float* x, const Geom& g) {
+  return g.Hx % 4 == 0 && g.H % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+}
+
+bool bp0_vec4(const float* y, const float* x, const Geom& g) {
+  return bp0_vec_in(y, g) && bp0_vec_out(x, g);
+}
+
+// Whether the run launches go (the default's epilogue also writes by single
+// heights, so rows of x need not be float4).
+bool bp0_runs(const float* y, const float* x, const Geom& g) {
+  const int v = kernel_variant(OP_BACKWARD_Z0);
+  return v == 0 ? bp0_vec_in(y, g) : bp0_vec4(y, x, g) && (v < 1 || v > 5);
+}
+
 // Both class launches for the voxel rows [row_lo, row_hi); row_lo is a
 // multiple of RUN (class-1 runs span RUN rows).
 // With addend, the class-1 launch also adds addend (same layout as x) into the
@@ -440,7 +461,7 @@ cudaError_t launch_bp_z0_runs_tma(const float* y, float* x, const float* angles,
 // same call (launch_ex); the class-1 launch follows the class-0 one.
 // addend_ready: an event the class-1 launch, which reads addend, waits for
 // (the class-0 launch runs before the addend is in).
-template <int R, bool FULL = false>
+template <int R, bool FULL = false, bool VOUT = true>
 cudaError_t launch_bp_z0_runs_h(const float* y, float* x, const float* angles, const Geom& g,
                                 int row_lo, int row_hi, cudaStream_t stream,
                                 const float* addend = nullptr, bool programmatic = false,
@@ -456,10 +477,10 @@ cudaError_t launch_bp_z0_runs_h(const float* y, float* x, const float* angles, c
     const dim3 grid(ceil_div(e0 - b0, BPR_WARPS), hchunks);
     cudaError_t e =
         programmatic
-            ? launch_ex(bp_z0_runs_kernel<0, R, false, FULL, true>, grid, block, 0, stream,
+            ? launch_ex(bp_z0_runs_kernel<0, R, false, FULL, true, VOUT>, grid, block, 0, stream,
                         true, y, x, angles, g, nmaj0, (int)b0, (int)e0, row_hi, g.accumulate,
                         no_addend)
-            : launch_ex(bp_z0_runs_kernel<0, R, false, FULL, false>, grid, block, 0, stream,
+            : launch_ex(bp_z0_runs_kernel<0, R, false, FULL, false, VOUT>, grid, block, 0, stream,
                         false, y, x, angles, g, nmaj0, (int)b0, (int)e0, row_hi, g.accumulate,
                         no_addend);
     if (e == cudaSuccess) e = cudaGetLastError();
@@ -478,7 +499,8 @@ cudaError_t launch_bp_z0_runs_h(const float* y, float* x, const float* angles, c
       if (e != cudaSuccess) return e;
       programmatic = false;
     }
-    if (addend)
+    // (containers come in whole float4: backward_z0_rows_can_add)
+    if (VOUT && addend)
       e = programmatic ? launch_ex(bp_z0_runs_kernel<1, R, true, FULL, true>, grid, block, 0,
                                    stream, true, y, x, angles, g, g.SX, (int)b1, (int)e1,
                                    row_hi, 1, addend)
@@ -486,10 +508,10 @@ cudaError_t launch_bp_z0_runs_h(const float* y, float* x, const float* angles, c
                                    stream, false, y, x, angles, g, g.SX, (int)b1, (int)e1,
                                    row_hi, 1, addend);
     else
-      e = programmatic ? launch_ex(bp_z0_runs_kernel<1, R, false, FULL, true>, grid, block, 0,
+      e = programmatic ? launch_ex(bp_z0_runs_kernel<1, R, false, FULL, true, VOUT>, grid, block, 0,
                                    stream, true, y, x, angles, g, g.SX, (int)b1, (int)e1,
                                    row_hi, 1, no_addend)
-                       : launch_ex(bp_z0_runs_kernel<1, R, false, FULL, false>, grid, block,
+                       : launch_ex(bp_z0_runs_kernel<1, R, false, FULL, false, VOUT>, grid, block,
                                    0, stream, false, y, x, angles, g, g.SX, (int)b1, (int)e1,
                                    row_hi, 1, no_addend);
     if (e == cudaSuccess) e = cudaGetLastError();
@@ -505,6 +527,9 @@ cudaError_t launch_bp_z0_runs(const float* y, float* x, const float* angles, con
                               int row_lo, int row_hi, cudaStream_t stream,
                               const float* addend = nullptr, bool programmatic = false,
                               cudaEvent_t addend_ready = nullptr) {
+  if (!bp0_vec_out(x, g))
+    return launch_bp_z0_runs_h<R, false, false>(y, x, angles, g, row_lo, row_hi, stream, nullptr,
+                                                programmatic, nullptr);
   if (R == 8 && g.H % (32 * 8) == 0)
     return launch_bp_z0_runs_h<R, true>(y, x, angles, g, row_lo, row_hi, stream, addend,
                                         programmatic, addend_ready);
@@ -541,14 +566,9 @@ cudaError_t launch_bp_z0_runs_split(const float* y, float* x, const float* angle
                               H8 > 0 ? nullptr : addend_ready);
 }
 
-bool bp0_vec4(const float* y, const float* x, const Geom& g) {
-  return (g.Hx % 4 == 0) && (g.Hy % 4 == 0) &&
-         ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
-}
-
 int launches_backward_z0(const float* y, const float* x, const Geom& g) {
   const int v = kernel_variant(OP_BACKWARD_Z0);
-  if (!bp0_vec4(y, x, g) || (v >= 1 && v <= 5)) return 1;
+  if (!bp0_runs(y, x, g)) return 1;
   const int H8 = bp0_split(g);  // runs: two launches per height part
   return (v != 6 && H8 > 0 && H8 < g.H) ? 4 : 2;
 }
@@ -565,6 +585,8 @@ cudaError_t launch_backward_z0(const float* y, float* x, const float* angles, co
                                cudaStream_t stream) {
   const bool vec4 = bp0_vec4(y, x, g);
   const int variant = kernel_variant(OP_BACKWARD_Z0);
+  if (variant == 0 && bp0_runs(y, x, g))
+    return launch_bp_z0_runs_split(y, x, angles, g, 0, g.SY, stream);
   if (vec4 && variant != 1) {
     switch (variant) {
       case 2: return launch_bp_z0_block<4, 4>(y, x, angles, g, stream);
@@ -593,8 +615,7 @@ unsigned long long wait_timeouts() {
 }
 
 int backward_z0_row_step(const float* y, const float* x, const Geom& g) {
-  const int v = kernel_variant(OP_BACKWARD_Z0);
-  return (bp0_vec4(y, x, g) && (v < 1 || v > 5)) ? RUN : 0;
+  return bp0_runs(y, x, g) ? RUN : 0;
 }
 
 cudaError_t launch_backward_z0_rows(const float* y, float* x, const float* angles,

@@ -159,8 +159,10 @@ __device__ __forceinline__ RunEntry run_entry(const float* angles, int a, const 
 // (BPR_CHUNK entries) and alist (BPR_LIST ints) are this warp's shared
 // tables.  All 32 lanes must call it together.  wait() runs (by the whole
 // warp) just before the outputs are written; with Wait::coherent the read of
-// the output bypasses L1.
-template <int PASS, int R = 4, class Wait = NoWait, bool ADD = false, bool FULL = false>
+// the output bypasses L1.  VOUT: x's rows take float4 stores (else single
+// heights; y's rows are 16-byte aligned all the same).
+template <int PASS, int R = 4, class Wait = NoWait, bool ADD = false, bool FULL = false,
+          bool VOUT = true>
 __device__ __forceinline__ void bp_runs_warp(const float* __restrict__ y, float* __restrict__ x,
                                              const float* __restrict__ angles, const Geom& g,
                                              int xi0, int yi0, int h, int accumulate,
@@ -258,9 +260,11 @@ __device__ __forceinline__ void bp_runs_warp(const float* __restrict__ y, float*
     for (int m = 0; m < RUN; ++m) {
       const int xi = xi0 + m * dx;
       const int yi = yi0 + m * dy;
-      if (xi < g.SX && yi < g.SY)
-        store_lane<R, Wait::coherent>(x + ((size_t)yi * g.SX + xi) * g.Hx, lh, acc[m],
-                                      accumulate);
+      if (xi < g.SX && yi < g.SY) {
+        float* row = x + ((size_t)yi * g.SX + xi) * g.Hx;
+        if constexpr (VOUT) store_lane<R, Wait::coherent>(row, lh, acc[m], accumulate);
+        else store_lane_heights<R, Wait::coherent>(row, lh, acc[m], accumulate, g.H);
+      }
     }
   }
 }

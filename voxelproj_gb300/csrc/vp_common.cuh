@@ -304,6 +304,26 @@ __device__ __forceinline__ void store_lane(float* p, const LaneH<R>& lh,
   }
 }
 
+// As store_lane, by single heights below H: for output rows that are not 16-byte
+// aligned or a height count that is not a multiple of 4.
+template <int R, bool COHERENT = false>
+__device__ __forceinline__ void store_lane_heights(float* p, const LaneH<R>& lh,
+                                                   const typename Vec<R>::T& v, int accumulate,
+                                                   int H) {
+  const float* parts = reinterpret_cast<const float*>(&v);
+#pragma unroll
+  for (int k = 0; k < LaneH<R>::NQ; ++k) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int h = lh.h + k * kSecondHalf + i;
+      if (h < H) {
+        if constexpr (COHERENT) store_out_coherent(p + h, parts[4 * k + i], accumulate);
+        else store_out(p + h, parts[4 * k + i], accumulate);
+      }
+    }
+  }
+}
+
 // One lane's heights of the output row at p: p = (p + v) + a when with_v,
 // else p = p + a (a: the addend row, same layout).
 template <int R>

@@ -47,8 +47,9 @@ using namespace detail;
 // gather half of the slab's major lines each: twice the blocks, each half as
 // long, so the last wave of a launch leaves less of the GPU idle.  The first
 // half writes (in the caller's mode); after a block barrier the second adds.
+// VOUT: see fp_z0_warp.
 template <int R, int KW, bool AGROUP, int UN, bool SPLIT = false, bool FULL = false,
-          bool PDL = false>
+          bool PDL = false, bool VOUT = true>
 __global__ void __launch_bounds__(32 * FP0_WARPS,
                                   SPLIT ? (R == 8 ? 7 : 8)
                                         : (R == 8 && KW == 4 ? (UN == 3 ? 6 : 7) : 0))
@@ -68,8 +69,9 @@ __global__ void __launch_bounds__(32 * FP0_WARPS,
     const bool second = w >= 2;
     const Slab hs = second ? Slab{ym, slab.y_hi, xm, slab.x_hi, slab.yy_lo, slab.yy_hi}
                            : Slab{slab.y_lo, ym, slab.x_lo, xm, slab.yy_lo, slab.yy_hi};
-    fp_z0_warp<R, KW, UN>(x, y, angles, g, p0, a, h, hs, second ? 1 : accumulate, cand[w],
-                          HalfBarrier{second});
+    fp_z0_warp<R, KW, UN, HalfBarrier, false, VOUT>(x, y, angles, g, p0, a, h, hs,
+                                                    second ? 1 : accumulate, cand[w],
+                                                    HalfBarrier{second});
     if (!second) __syncthreads();  // the second half adds after this one wrote
   } else {
     // a programmatic launch of the next slab may start as this one's last
@@ -78,7 +80,7 @@ __global__ void __launch_bounds__(32 * FP0_WARPS,
     const int p0 = (AGROUP ? blockIdx.x : blockIdx.x * FP0_WARPS + w) * KW;
     const int a = a_base + (AGROUP ? blockIdx.y * FP0_WARPS + w : blockIdx.y);
     using Wait = std::conditional_t<PDL, PdlWait, NoWait>;
-    fp_z0_warp<R, KW, UN, Wait, FULL>(x, y, angles, g, p0, a, h, slab, accumulate, cand[w]);
+    fp_z0_warp<R, KW, UN, Wait, FULL, VOUT>(x, y, angles, g, p0, a, h, slab, accumulate, cand[w]);
   }
 }
 
@@ -359,9 +361,18 @@ Slab fp0_slab(const Geom& g, const Fp0Config& c, int k, int n) {
   return slab_of(k, c.cls, wy, wx, g.SY, g.SX);
 }
 
+// Rows of x take float4 loads; rows of y float4 stores.
+bool fp0_vec_in(const float* x, const Geom& g) {
+  return g.Hx % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+}
+bool fp0_vec_out(const float* y, const Geom& g) {
+  return g.Hy % 4 == 0 && g.H % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+}
+
+// Whether the float4 kernels run: both sides in float4, or the loads alone in
+// the default's forms, which have epilogues by single heights.
 bool fp0_vec4(const float* x, const float* y, const Geom& g) {
-  return (g.Hx % 4 == 0) && (g.Hy % 4 == 0) &&
-         ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  return fp0_vec_in(x, g) && (fp0_vec_out(y, g) || kernel_variant(OP_FORWARD_Z0) == 0);
 }
 
 int launches_forward_z0(const float* x, const float* y, const Geom& g);
@@ -384,9 +395,11 @@ struct SlabLaunch {
   // the launch directly follows this call's previous slab launch on the
   // stream: it may start while that one runs (launch_ex)
   bool programmatic = false;
+  bool vec_out = true;  // fp0_vec_out
 };
 
-template <int R, int KW, bool AGROUP, int UN, bool SPLIT = false, bool FULL = false>
+template <int R, int KW, bool AGROUP, int UN, bool SPLIT = false, bool FULL = false,
+          bool VOUT = true>
 cudaError_t launch_slab(const SlabLaunch& L, cudaStream_t stream, int* launches) {
   dim3 block(32, FP0_WARPS);
   const long long per_launch = AGROUP ? (long long)kMaxGridYZ * FP0_WARPS : kMaxGridYZ;
@@ -406,13 +419,13 @@ cudaError_t launch_slab(const SlabLaunch& L, cudaStream_t stream, int* launches)
     cudaError_t e;
     if constexpr (kPdlForm) {
       if (L.programmatic || a_base > L.a_lo)
-        e = launch_ex(fp_z0_kernel<R, KW, AGROUP, UN, SPLIT, FULL, true>, grid, block, 0, stream,
+        e = launch_ex(fp_z0_kernel<R, KW, AGROUP, UN, SPLIT, FULL, true, VOUT>, grid, block, 0, stream,
                       true, L.x, L.y, L.angles, g, (int)a_base, L.slab, L.accumulate);
       else
-        e = launch_ex(fp_z0_kernel<R, KW, AGROUP, UN, SPLIT, FULL, false>, grid, block, 0,
+        e = launch_ex(fp_z0_kernel<R, KW, AGROUP, UN, SPLIT, FULL, false, VOUT>, grid, block, 0,
                       stream, false, L.x, L.y, L.angles, g, (int)a_base, L.slab, L.accumulate);
     } else {
-      e = launch_ex(fp_z0_kernel<R, KW, AGROUP, UN, SPLIT, FULL, false>, grid, block, 0, stream,
+      e = launch_ex(fp_z0_kernel<R, KW, AGROUP, UN, SPLIT, FULL, false, VOUT>, grid, block, 0, stream,
                     false, L.x, L.y, L.angles, g, (int)a_base, L.slab, L.accumulate);
     }
     if (launches) ++*launches;
@@ -515,6 +528,11 @@ cudaError_t launch_slab_aligned(const SlabLaunch& L, cudaStream_t stream, int* l
 }
 
 cudaError_t launch_slab_config(const Fp0Config& c, const SlabLaunch& L, cudaStream_t s, int* n) {
+  if (!L.vec_out && c.R != 1) {  // the default's forms (fp0_vec4)
+    if (c.R == 8) return launch_slab<8, 4, true, 2, false, false, false>(L, s, n);
+    if (c.split) return launch_slab<4, 4, false, FP0_UNROLL, true, false, false>(L, s, n);
+    return launch_slab<4, 4, false, FP0_UNROLL, false, false, false>(L, s, n);
+  }
   if (c.R == 8 && c.staged) {
     const bool full = L.g.H % 256 == 0;
     if (c.staged == 2)
@@ -554,7 +572,7 @@ cudaError_t launch_fp_z0_config(const float* x, float* y, const float* angles, c
   const int nslabs = fp0_slabs(g, c);
   for (int k = k0; k < k1 && k < nslabs; ++k) {
     const SlabLaunch L{x, y, angles, g, fp0_slab(g, c, k, nslabs), k == 0 ? g.accumulate : 1,
-                       0, g.n_ang, k > k0};
+                       0, g.n_ang, k > k0, fp0_vec_out(y, g)};
     const cudaError_t e = launch_slab_config(c, L, stream, launches);
     if (e != cudaSuccess) return e;
   }
@@ -669,7 +687,7 @@ cudaError_t launch_forward_z0_stream(const float* x, float* y, const float* angl
   Fp0Config c = fp0_config(gm, vec4, v);
   c.cls = true;
   const SlabLaunch L{x, y, angles, gm, Slab{rows_lo, rows_hi, cols_lo, cols_hi, 0, g.SY},
-                     accumulate, a_lo, a_hi};
+                     accumulate, a_lo, a_hi, false, fp0_vec_out(y, gm)};
   return launch_slab_config(c, L, stream, launches);
 }
 

@@ -138,11 +138,13 @@ __host__ __device__ inline Slab slab_of(int k, bool cls, int wy, int wx, int SY,
 // One warp: angle a, bins [p0, p0 + nb) (nb <= KW), this lane's heights from h (LaneH:
 // R = 8 is [h, h + 4) and [h + 128, h + 132)), the voxels of slab s.  FULL:
 // every lane's heights are inside [0, H).
-// UN candidates are loaded together.  cand is this warp's shared candidate list of
+// UN candidates are loaded together.  VOUT: y's rows take float4 stores (else
+// single heights, R = 4 or 8 all the same: x's rows are 16-byte aligned).  cand is this warp's shared candidate list of
 // Fp0Cap<KW>::list entries.  All 32 lanes must call it together.
 // wait() runs (by the whole warp) just before the outputs are written; with
 // Wait::coherent the read of the output bypasses L1.
-template <int R, int KW, int UN = FP0_UNROLL, class Wait = NoWait, bool FULL = false>
+template <int R, int KW, int UN = FP0_UNROLL, class Wait = NoWait, bool FULL = false,
+          bool VOUT = true>
 __device__ __forceinline__ void fp_z0_warp(const float* __restrict__ x, float* __restrict__ y,
                                            const float* __restrict__ angles, const Geom& g,
                                            int p0, int a, int h, const Slab& s,
@@ -239,8 +241,11 @@ __device__ __forceinline__ void fp_z0_warp(const float* __restrict__ x, float* _
 #pragma unroll
   for (int b = 0; b < KW; ++b) {
     const int p = p0 + b;
-    if (p < g.PX && b < nb)
-      store_lane<R, Wait::coherent>(y + ((size_t)a * g.PX + p) * g.Hy, lh, acc[b], accumulate);
+    if (p < g.PX && b < nb) {
+      float* row = y + ((size_t)a * g.PX + p) * g.Hy;
+      if constexpr (VOUT) store_lane<R, Wait::coherent>(row, lh, acc[b], accumulate);
+      else store_lane_heights<R, Wait::coherent>(row, lh, acc[b], accumulate, g.H);
+    }
   }
 }
 

@@ -55,6 +55,11 @@ enum Op : int { OP_FORWARD_Z0 = 0, OP_BACKWARD_Z0 = 1, OP_FORWARD_Z2 = 2, OP_BAC
                 OP_COUNT = 4 };
 int kernel_variant(int op);
 
+// dst rows of Hd floats from src rows of Hs: heights [0, H), then zeros; dst
+// 16-byte aligned, Hd a multiple of 4 (vp_z2.cu).
+cudaError_t pad_heights(const float* src, float* dst, long long rows, int Hs, int Hd, int H,
+                        cudaStream_t stream);
+
 // z_order 2 through the z_order 0 kernels (vp_z2.cu).
 bool z2_uses_transpose(const Geom& g);
 size_t z2_workspace_bytes(const Geom& g);

@@ -120,7 +120,37 @@ cudaError_t transpose(const float* src, float* dst, long long rows, long long co
 
 inline long long round4(long long v) { return (v + 3) / 4 * 4; }
 
+// dst rows of Hd floats (16-byte aligned) from src rows of Hs: heights [0, H),
+// then zeros.  blockDim.x lanes share a row, a float4 of it each per step.
+__global__ void __launch_bounds__(256)
+    pad_kernel(const float* __restrict__ src, float* __restrict__ dst, long long rows, int Hs,
+               int Hd, int H) {
+  const int nq = Hd / 4;
+  for (long long r = (long long)blockIdx.x * blockDim.y + threadIdx.y; r < rows;
+       r += (long long)gridDim.x * blockDim.y) {
+    const float* s = src + r * Hs;
+    float4* d = reinterpret_cast<float4*>(dst + r * Hd);
+    for (int q = threadIdx.x; q < nq; q += blockDim.x) {
+      float v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = 4 * q + i < H ? __ldg(s + 4 * q + i) : 0.0f;
+      d[q] = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  }
+}
+
 }  // namespace
+
+cudaError_t pad_heights(const float* src, float* dst, long long rows, int Hs, int Hd, int H,
+                        cudaStream_t stream) {
+  int tx = 32;
+  while (tx > 1 && tx / 2 >= Hd / 4) tx /= 2;
+  const int ty = 256 / tx;
+  const long long blocks = (rows + ty - 1) / ty;
+  pad_kernel<<<(unsigned)(blocks < 8192 ? blocks : 8192), dim3(tx, ty), 0, stream>>>(
+      src, dst, rows, Hs, Hd, H);
+  return cudaGetLastError();
+}
 
 bool z2_uses_transpose(const Geom& g) { return g.H >= 32; }
 
