@@ -273,7 +273,8 @@ __global__ void __launch_bounds__(TMA_THREADS, 4)
 }
 
 // ---------------------------------------------------------------------------
-// z_order 2: x (H, SY, SX), y (H, n_ang, PX); x / PX are contiguous.
+// z_order 2 in the reference's order of additions (with variant 4), below 32
+// heights: x (H, SY, SX), y (H, n_ang, PX); x / PX are contiguous.
 // A thread owns one voxel column (lane <-> xi, so loads and stores coalesce
 // along x) and BP2_RH heights.  Weights are per thread (lanes hold different
 // voxels) and are reused across the thread's heights.  Angle constants for a
@@ -450,7 +451,7 @@ bool bp0_vec4(const float* y, const float* x, const Geom& g) {
 // heights, so rows of x need not be float4).
 bool bp0_runs(const float* y, const float* x, const Geom& g) {
   const int v = kernel_variant(OP_BACKWARD_Z0);
-  return v == 0 ? bp0_vec_in(y, g) : bp0_vec4(y, x, g) && (v < 1 || v > 5);
+  return v == 0 ? bp0_vec_in(y, g) && !z0_backward_thin(g) : bp0_vec4(y, x, g) && (v < 1 || v > 5);
 }
 
 // Both class launches for the voxel rows [row_lo, row_hi); row_lo is a
@@ -585,6 +586,7 @@ cudaError_t launch_backward_z0(const float* y, float* x, const float* angles, co
                                cudaStream_t stream) {
   const bool vec4 = bp0_vec4(y, x, g);
   const int variant = kernel_variant(OP_BACKWARD_Z0);
+  if (variant == 0 && z0_backward_thin(g)) return launch_backward_thin(y, x, angles, g, 0, stream);
   if (variant == 0 && bp0_runs(y, x, g))
     return launch_bp_z0_runs_split(y, x, angles, g, 0, g.SY, stream);
   if (vec4 && variant != 1) {
@@ -647,6 +649,9 @@ cudaError_t launch_backward_z0_rows_add(const float* y, float* x, const float* a
 
 cudaError_t launch_backward_z2(const float* y, float* x, const float* angles, const Geom& g,
                                cudaStream_t stream) {
+  // (the reference's order of additions goes with the z_order 0 variant that has it)
+  if (kernel_variant(OP_BACKWARD_Z0) != 4)
+    return launch_backward_thin(y, x, angles, g, 2, stream);
   dim3 block(32, BP2_WARPS);
   dim3 grid(ceil_div(g.SX, 32), ceil_div(g.SY, BP2_WARPS), ceil_div(g.H, BP2_RH));
   bp_z2_kernel<<<grid, block, 0, stream>>>(y, x, angles, g);

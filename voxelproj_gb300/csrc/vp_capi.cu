@@ -355,7 +355,7 @@ namespace {
 int run_z2(bool forward, const float* in, float* out, const float* angles, const vp::Geom& g,
            void* ws, size_t ws_bytes, cudaStream_t stream) {
   if (!vp::z2_uses_transpose(g)) {
-    cudaError_t e = forward ? vp::launch_forward_z2(in, out, angles, g, stream)
+    cudaError_t e = forward ? vp::launch_forward_thin(in, out, angles, g, 2, stream)
                             : vp::launch_backward_z2(in, out, angles, g, stream);
     return finish(e, vp::launches_z2(g, forward));
   }

@@ -115,11 +115,6 @@ __device__ __forceinline__ BinWeights weights_from_offset(int r, float xv, const
   return o;
 }
 
-__device__ __forceinline__ BinWeights bin_weights(float xp, const AngleConst& k) {
-  const int r = __float2int_rn(xp);
-  return weights_from_offset(r, (float)r - xp, k);
-}
-
 // Error-free sum: s + e == a + b exactly (Knuth's TwoSum).
 __device__ __forceinline__ float two_sum(float a, float b, float& e) {
   const float s = __fadd_rn(a, b);
@@ -128,14 +123,13 @@ __device__ __forceinline__ float two_sum(float a, float b, float& e) {
   return s;
 }
 
-// Weights with the sub-bin offset xv = r - xp evaluated from an unrounded xp:
+// r = round(xp) and the sub-bin offset xv = r - xp from an unrounded xp:
 // the products and sums of xp are carried as (value, error) pairs with FMA
 // and TwoSum, so at 512^3 the offset is not limited by the ~3e-5 px spacing
 // of floats near 256.  Used by TRIG_PRECISE; TRIG_REF keeps the plain formula
 // so that it rounds the way the reference does.
-__device__ __forceinline__ BinWeights bin_weights_compensated(float relx, float rely,
-                                                              const AngleConst& k,
-                                                              float pcent) {
+__device__ __forceinline__ int compensated_offset(float relx, float rely, const AngleConst& k,
+                                                  float pcent, float* xv) {
   const float p1 = __fmul_rn(relx, k.c);
   const float e1 = fmaf(relx, k.c, -p1);
   const float p2 = __fmul_rn(rely, k.s);
@@ -145,15 +139,27 @@ __device__ __forceinline__ BinWeights bin_weights_compensated(float relx, float 
   const float hi = two_sum(s1, pcent, e4);
   const float lo = (e1 + e2) + (e3 + e4);
   const int r = __float2int_rn(hi);
-  const float xv = __fsub_rn((float)r, hi) - lo;
-  return weights_from_offset(r, xv, k);
+  *xv = __fsub_rn((float)r, hi) - lo;
+  return r;
+}
+
+// The bin r = round(xp) of voxel (relx, rely) at one angle and its sub-bin
+// offset xv = r - xp.
+__device__ __forceinline__ int voxel_offset(float relx, float rely, const AngleConst& k,
+                                            float pcent, int trig, float* xv) {
+  if (trig == TRIG_PRECISE) return compensated_offset(relx, rely, k, pcent, xv);
+  const float xp = det_coord(relx, rely, k.c, k.s, pcent);
+  const int r = __float2int_rn(xp);
+  *xv = (float)r - xp;
+  return r;
 }
 
 // The weights of voxel (relx, rely) at one angle, in the given trig mode.
 __device__ __forceinline__ BinWeights voxel_weights(float relx, float rely, const AngleConst& k,
                                                     float pcent, int trig) {
-  if (trig == TRIG_PRECISE) return bin_weights_compensated(relx, rely, k, pcent);
-  return bin_weights(det_coord(relx, rely, k.c, k.s, pcent), k);
+  float xv;
+  const int r = voxel_offset(relx, rely, k, pcent, trig, &xv);
+  return weights_from_offset(r, xv, k);
 }
 
 // acc + w * v per component, two components per instruction: the packed

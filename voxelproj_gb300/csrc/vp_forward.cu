@@ -8,7 +8,7 @@
 // (angle, bin) gathers exactly the voxels whose three-bin footprint reaches
 // it, with the same closed-form weights the adjoint uses, so A and A^T are
 // the same matrix up to float summation order:
-//   weight of bin p from voxel v = w_{p - round(xp_v) + 1}(v)   (bin_weights).
+//   weight of bin p from voxel v = w_{p - round(xp_v) + 1}(v)   (voxel_weights).
 //
 // Voxel enumeration: along the axis whose unit step moves xp by less
 // ("major"), every index is visited; along the other ("minor", |shift| >=
@@ -143,72 +143,6 @@ __global__ void __launch_bounds__(32 * FPS_WARPS, 7)
   }
   fps_plain_block<FULL>(x, y, angles, g, slab, accumulate, a0, h0, bx, -E,
                         (int)gridDim.x - 1 - E, G, cand[w]);
-}
-
-// ---------------------------------------------------------------------------
-// z_order 2: x (H, SY, SX), y (H, n_ang, PX); SX / PX contiguous.
-// A thread owns one bin p (lane <-> p, so the output row is coalesced) of one
-// angle and FP2_RH heights, walks the major axis, and gathers the candidate
-// voxels of its bin; each weight is reused across the thread's heights.
-// ---------------------------------------------------------------------------
-constexpr int FP2_RH = 8;
-constexpr int FP2_WARPS = 4;
-
-__global__ void __launch_bounds__(32 * FP2_WARPS)
-    fp_z2_kernel(const float* __restrict__ x, float* __restrict__ y,
-                 const float* __restrict__ angles, Geom g, int a_base) {
-  const int lane = threadIdx.x;
-  const int w = threadIdx.y;
-  const int p = blockIdx.x * 32 + lane;
-  const int a = a_base + blockIdx.y * FP2_WARPS + w;
-  const int h0 = blockIdx.z * FP2_RH;
-  if (a >= g.n_ang) return;  // warp-uniform
-  const bool pv = p < g.PX;
-
-  const AngleConst k = angle_const(__ldg(angles + a), g.trig);
-  const bool minor_x = fabsf(k.c) >= fabsf(k.s);
-  const int n_major = minor_x ? g.SY : g.SX;
-  const int n_minor = minor_x ? g.SX : g.SY;
-  const float cent_major = minor_x ? g.ycent : g.xcent;
-  const float cent_minor = minor_x ? g.xcent : g.ycent;
-  const float sh_major = minor_x ? k.s : k.c;
-  const float inv_sh_minor = 1.0f / (minor_x ? k.c : k.s);
-  const float t_lo = (float)p - 0.5f - k.b - kWindowMargin;
-  const float t_hi = (float)p + 0.5f + k.b + kWindowMargin;
-  const size_t xh_stride = (size_t)g.SY * g.SX;
-
-  float acc[FP2_RH];
-#pragma unroll
-  for (int i = 0; i < FP2_RH; ++i) acc[i] = 0.0f;
-
-  if (pv) {
-    for (int i = 0; i < n_major; ++i) {
-      const MinorRange mr = minor_range(i, cent_major, sh_major, cent_minor, inv_sh_minor,
-                                        0, n_minor - 1, g.pcent, t_lo, t_hi);
-      for (int m = mr.lo; m <= mr.hi; ++m) {
-        const int xi = minor_x ? m : i;
-        const int yi = minor_x ? i : m;
-        const BinWeights bw =
-            voxel_weights((float)xi - g.xcent, (float)yi - g.ycent, k, g.pcent, g.trig);
-        const int q = p - bw.r + 1;
-        const float wt = (q == 0) ? bw.w0 : (q == 1) ? bw.w1 : (q == 2) ? bw.w2 : 0.0f;
-        if (wt != 0.0f) {
-          const float* px = x + (size_t)yi * g.SX + xi;
-#pragma unroll
-          for (int r = 0; r < FP2_RH; ++r) {
-            const int h = h0 + r;
-            if (h < g.H) acc[r] = fmaf(wt, __ldg(px + (size_t)h * xh_stride), acc[r]);
-          }
-        }
-      }
-    }
-    const size_t yh_stride = (size_t)g.n_ang * g.PX;
-#pragma unroll
-    for (int r = 0; r < FP2_RH; ++r) {
-      const int h = h0 + r;
-      if (h < g.H) store_out(y + (size_t)h * yh_stride + (size_t)a * g.PX + p, acc[r], g.accumulate);
-    }
-  }
 }
 
 inline unsigned ceil_div(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
@@ -376,10 +310,6 @@ bool fp0_vec4(const float* x, const float* y, const Geom& g) {
 }
 
 int launches_forward_z0(const float* x, const float* y, const Geom& g);
-
-int launches_forward_z2(const Geom& g) {
-  return (int)ceil_div(g.n_ang, (long long)kMaxGridYZ * FP2_WARPS);
-}
 
 // One slab launch: slab, the caller's mode for it, and the angles [a_lo, a_hi)
 // (the kernels index angles and y absolutely; g.n_ang is set to a_hi for
@@ -605,6 +535,7 @@ cudaError_t launch_forward_z0(const float* x, float* y, const float* angles, con
                               cudaStream_t stream) {
   const bool vec4 = fp0_vec4(x, y, g);
   const int v = kernel_variant(OP_FORWARD_Z0);
+  if (v == 0 && z0_forward_thin(g)) return launch_forward_thin(x, y, angles, g, 0, stream);
   const HeightParts hp = fp0_parts(g, vec4, v);
   for (int i = 0; i < hp.n; ++i) {
     const Fp0Config c = fp0_config(hp.g[i], vec4, v);
@@ -633,6 +564,7 @@ Fp0Plan forward_z0_plan(const Geom& g, bool vec4, int variant) {
 int launches_forward_z0(const float* x, const float* y, const Geom& g) {
   const bool vec4 = fp0_vec4(x, y, g);
   const int v = kernel_variant(OP_FORWARD_Z0);
+  if (v == 0 && z0_forward_thin(g)) return launches_forward_thin(g);
   const HeightParts hp = fp0_parts(g, vec4, v);
   int n = 0;
   for (int i = 0; i < hp.n; ++i) {
@@ -699,20 +631,6 @@ cudaError_t launch_forward_z0_rest(const float* x, float* y, const float* angles
   const Fp0Config c = fp0_config(hp.g[1], vec4, kernel_variant(OP_FORWARD_Z0));
   return launch_fp_z0_config(x + hp.h0[1], y + hp.h0[1], angles, hp.g[1], c, 0, 1 << 30,
                              stream, launches);
-}
-
-cudaError_t launch_forward_z2(const float* x, float* y, const float* angles, const Geom& g,
-                              cudaStream_t stream) {
-  dim3 block(32, FP2_WARPS);
-  const long long per_launch = (long long)kMaxGridYZ * FP2_WARPS;
-  for (long long a_base = 0; a_base < g.n_ang; a_base += per_launch) {
-    const long long na = g.n_ang - a_base < per_launch ? g.n_ang - a_base : per_launch;
-    dim3 grid(ceil_div(g.PX, 32), ceil_div(na, FP2_WARPS), ceil_div(g.H, FP2_RH));
-    fp_z2_kernel<<<grid, block, 0, stream>>>(x, y, angles, g, (int)a_base);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
 }
 
 }  // namespace vp

@@ -826,7 +826,7 @@ cudaError_t z2_host(bool forward, const float* in_host, float* out_host, const f
                                s));
       else
         VP_TRY(cudaMemsetAsync(ys, 0, (size_t)H * bins * sizeof(float), s));
-      VP_TRY(launch_forward_z2(xs, ys, ad, gk, s));
+      VP_TRY(launch_forward_thin(xs, ys, ad, gk, 2, s));
       *launches += launches_z2(gk, true);
       VP_TRY(cudaMemcpyAsync(y_host, ys, (size_t)H * bins * sizeof(float), cudaMemcpyDefault, s));
     }

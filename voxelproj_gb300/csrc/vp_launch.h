@@ -36,8 +36,6 @@ cudaError_t launch_ex(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem,
 // y (z_order 0: (n_ang, PX, Hy), z_order 2: (Hy, n_ang, PX)) += A x.
 cudaError_t launch_forward_z0(const float* x, float* y, const float* angles, const Geom& g,
                               cudaStream_t stream);
-cudaError_t launch_forward_z2(const float* x, float* y, const float* angles, const Geom& g,
-                              cudaStream_t stream);
 // x (z_order 0: (SY, SX, Hx), z_order 2: (Hx, SY, SX)) += A^T y.
 cudaError_t launch_backward_z0(const float* y, float* x, const float* angles, const Geom& g,
                                cudaStream_t stream);
@@ -54,6 +52,21 @@ void count_launches(int n);
 enum Op : int { OP_FORWARD_Z0 = 0, OP_BACKWARD_Z0 = 1, OP_FORWARD_Z2 = 2, OP_BACKWARD_Z2 = 3,
                 OP_COUNT = 4 };
 int kernel_variant(int op);
+
+// Few heights (vp_thin.cu): the arrays in z_order z.
+cudaError_t launch_forward_thin(const float* x, float* y, const float* angles, const Geom& g,
+                                int z, cudaStream_t stream);
+cudaError_t launch_backward_thin(const float* y, float* x, const float* angles, const Geom& g,
+                                 int z, cudaStream_t stream);
+int launches_forward_thin(const Geom& g);
+// The defaults take them in z_order 0 up to 8 heights, the adjoint only for
+// height counts that are not a multiple of 4 (it must equal the batched run
+// adjoint bit for bit on the others).  256 x 256, 180 angles, against the
+// scalar and 4-height kernels: A 455 -> 53 us (1 height), 573 -> 116 (4),
+// 582 -> 200 (8), but 583 -> 545 (16) and 477 -> 529 (19); A^T 363 -> 39 (1),
+// 367 -> 67 (3), 378 -> 107 (7), but 321 -> 644 (16).
+inline bool z0_forward_thin(const Geom& g) { return g.H <= 8; }
+inline bool z0_backward_thin(const Geom& g) { return g.H <= 7 && g.H % 4 != 0; }
 
 // dst rows of Hd floats from src rows of Hs: heights [0, H), then zeros; dst
 // 16-byte aligned, Hd a multiple of 4 (vp_z2.cu).
@@ -176,6 +189,5 @@ cudaError_t z2_host(bool forward, const float* in_host, float* out_host, const f
 // split past 65535 angle blocks).
 int launches_forward_z0(const float* x, const float* y, const Geom& g);
 int launches_backward_z0(const float* y, const float* x, const Geom& g);
-int launches_forward_z2(const Geom& g);
 
 }  // namespace vp

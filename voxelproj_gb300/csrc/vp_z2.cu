@@ -161,7 +161,7 @@ size_t z2_workspace_bytes(const Geom& g) {
 }
 
 int launches_z2(const Geom& g, bool forward) {
-  if (!z2_uses_transpose(g)) return forward ? launches_forward_z2(g) : 1;
+  if (!z2_uses_transpose(g)) return forward ? launches_forward_thin(g) : 1;
   // the transposed path runs the z_order 0 kernels on 16-byte aligned scratch
   // with a height extent that is a multiple of 4
   Geom g0 = g;
