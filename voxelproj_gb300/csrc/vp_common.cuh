@@ -155,10 +155,16 @@ __device__ __forceinline__ int voxel_offset(float relx, float rely, const AngleC
 }
 
 // The weights of voxel (relx, rely) at one angle, in the given trig mode.
+// (Two separate evaluations: with voxel_offset's two modes joined before one
+// weights_from_offset the forward ran 2-5% slower.)
 __device__ __forceinline__ BinWeights voxel_weights(float relx, float rely, const AngleConst& k,
                                                     float pcent, int trig) {
   float xv;
-  const int r = voxel_offset(relx, rely, k, pcent, trig, &xv);
+  if (trig == TRIG_PRECISE) {
+    const int r = compensated_offset(relx, rely, k, pcent, &xv);
+    return weights_from_offset(r, xv, k);
+  }
+  const int r = voxel_offset(relx, rely, k, pcent, TRIG_REF, &xv);
   return weights_from_offset(r, xv, k);
 }
 
