@@ -144,10 +144,12 @@ VP_API int vp_backward_z2(const float* y, int64_t y0, int64_t y1, int64_t y2,
 /* z_order 2 with caller-supplied scratch.  For H >= 32 the z_order 2
  * operators transpose to height-fastest order, run the z_order 0 kernels and
  * transpose back (adding into the output); they need
- * vp_z2_workspace_bytes(...) bytes of device scratch (0 when H < 32).  The
+ * vp_z2_workspace_bytes(...) bytes of device scratch.  From 5 to 31
+ * heights the forward does so too where it gets the scratch, and runs without
+ * it otherwise; below 5 heights the size is 0.  The
  * plain vp_forward_z2 / vp_backward_z2 take it from a library-private
  * stream-ordered pool; these variants use `workspace` instead and fail with
- * VP_ERR_WORKSPACE if it is too small.  No counterpart in the reference,
+ * VP_ERR_WORKSPACE if it is too small for 32 heights or more.  No counterpart in the reference,
  * which staged its input through a per-call cudaArray. */
 VP_API size_t vp_z2_workspace_bytes(int64_t x0, int64_t x1, int64_t x2,
                                     int64_t y0, int64_t y1, int64_t y2);
@@ -165,8 +167,9 @@ VP_API int vp_backward_z2_ws(const float* y, int64_t y0, int64_t y1, int64_t y2,
  * hosts whose own allocator owns the device).  Same arguments and results as
  * vp_forward_z2, but its scratch is an array of VP_NOALLOC_SCRATCH_BYTES
  * (64 MiB) compiled into the library, held by every GPU that loads the
- * library until the process exits.  Problems needing more scratch than that
- * (vp_z2_workspace_bytes) return VP_ERR_SCRATCH_LIMIT and leave y unchanged.
+ * library until the process exits.  Problems of 32 heights or more that need
+ * more scratch than that (vp_z2_workspace_bytes) return VP_ERR_SCRATCH_LIMIT and
+ * leave y unchanged; with fewer heights they run without scratch.
  * The first call on a device looks up the array's address (make it before
  * any stream capture).  All calls share the array: calls that overlap on the
  * GPU race and must be ordered by the caller.  No counterpart in the

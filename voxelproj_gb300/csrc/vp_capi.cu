@@ -168,8 +168,8 @@ namespace {
 // epilogues write such outputs by single heights).  The copy costs one read
 // and one write of the input; the scalar kernels it replaces held one height
 // per lane: (301, 257, 203) and 181 angles, A 3.76 -> 1.16 ms, A^T 3.00 ->
-// 0.81 ms.  From 33 heights on: up to 32, one scalar chunk per warp does the
-// float4 form's work.  Not under stream capture, and not without memory for
+// 0.81 ms.  The adjoint from 33 heights on: up to 32, one scalar chunk per warp
+// does the float4 form's work.  Not under stream capture, and not without memory for
 // the copy: the scalar kernels run then, as they do for other variants.
 constexpr int kPadMinHeights = 33;
 
@@ -178,7 +178,8 @@ constexpr int kPadMinHeights = 33;
 cudaError_t padded_input(int op, const float* in, int64_t rows, int Hin, const vp::Geom& g,
                          cudaStream_t stream, float** copy, int* Hp) {
   *copy = nullptr;
-  if (vp::kernel_variant(op) != 0 || g.H < kPadMinHeights ||
+  if (vp::kernel_variant(op) != 0 ||
+      (op == vp::OP_FORWARD_Z0 ? vp::z0_forward_thin(g) : g.H < kPadMinHeights) ||
       (Hin % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0))
     return cudaSuccess;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -352,23 +353,43 @@ size_t vp_z2_workspace_bytes(int64_t x0, int64_t x1, int64_t x2, int64_t y0, int
 namespace {
 
 // z_order 2 dispatch shared by the entry points with and without workspace.
+// Below 32 heights the workspace is optional: without it (a smaller one given,
+// no room in the pool, or under capture, where the pool would add memory
+// nodes) the kernels for few heights run.
 int run_z2(bool forward, const float* in, float* out, const float* angles, const vp::Geom& g,
            void* ws, size_t ws_bytes, cudaStream_t stream) {
-  if (!vp::z2_uses_transpose(g)) {
-    cudaError_t e = forward ? vp::launch_forward_thin(in, out, angles, g, 2, stream)
-                            : vp::launch_backward_z2(in, out, angles, g, stream);
-    return finish(e, vp::launches_z2(g, forward));
-  }
   const size_t need = vp::z2_workspace_bytes(g);
+  const bool must = vp::z2_uses_transpose(g);
+  bool use = must || (forward && vp::z2_can_transpose(g));
+  if (use && ws != nullptr && ws_bytes < need) {
+    if (must) return VP_ERR_WORKSPACE;
+    use = false;
+  }
   bool owned = false;
-  if (ws == nullptr) {
-    cudaMemPool_t pool;
-    cudaError_t e = private_pool(&pool);
-    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&ws, need, pool, stream);
-    if (e != cudaSuccess) return finish(e, 0);
-    owned = true;
-  } else if (ws_bytes < need) {
-    return VP_ERR_WORKSPACE;
+  if (use && ws == nullptr) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!must) {
+      const cudaError_t e = cudaStreamIsCapturing(stream, &cap);
+      if (e != cudaSuccess) return finish(e, 0);
+    }
+    if (cap != cudaStreamCaptureStatusNone) {
+      use = false;
+    } else {
+      cudaMemPool_t pool;
+      cudaError_t e = private_pool(&pool);
+      if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&ws, need, pool, stream);
+      if (e != cudaSuccess && must) return finish(e, 0);
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        use = false;
+      }
+      owned = use;
+    }
+  }
+  if (!use) {
+    const cudaError_t e = forward ? vp::launch_forward_thin(in, out, angles, g, 2, stream)
+                                  : vp::launch_backward_z2(in, out, angles, g, stream);
+    return finish(e, forward ? vp::launches_forward_thin(g) : 1);
   }
   cudaError_t e = forward
       ? vp::forward_z2_transposed(in, out, angles, g, static_cast<float*>(ws), stream)
@@ -509,7 +530,8 @@ extern "C" int vp_forward_z2_noalloc(const float* x, int64_t x0, int64_t x1, int
     return s;
   if (empty) return VP_OK;
   const size_t need = vp::z2_workspace_bytes(g);
-  if (need > VP_NOALLOC_SCRATCH_BYTES) return VP_ERR_SCRATCH_LIMIT;
+  // (below 32 heights a problem past the array runs without scratch)
+  if (need > VP_NOALLOC_SCRATCH_BYTES && vp::z2_uses_transpose(g)) return VP_ERR_SCRATCH_LIMIT;
   float* scratch = nullptr;
   if (need > 0) {
     const cudaError_t e = noalloc_scratch(&scratch);

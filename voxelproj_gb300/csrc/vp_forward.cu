@@ -159,6 +159,7 @@ struct Fp0Config {
   int slab_mb;    // volume bytes of one height chunk per slab launch
   bool cls;       // class slabs (rows for one angle class, columns for the other)
   bool split;     // two warps per bin run, each on half of the major lines
+  int band;       // banded form (vp_fp_band.cuh): runs per warp, 0 = candidate lists
   int staged;     // aligned neighbouring-angle forms (vp_fp_staged.cuh), 8 heights per
                   // lane only: 1 = staged by tensor copies, 2 = plain loads; 0 = none
 };
@@ -187,15 +188,20 @@ struct Fp0Config {
 // the same bin layout; 8-height variants on problems of at most 128 heights
 // run the 4-height form.
 
-// Whether the default's 4-height form takes two warps per bin run (SPLIT),
-// for grids of less than two waves of blocks: when twice as many blocks of
-// half the work take fewer half-waves than the blocks take waves, or when
-// the blocks fill less than three quarters of one wave (smaller blocks then
-// balance the SMs better).  Measured A per call (192 angles, default /
-// split): 128^3 0.212 / 0.188 ms (1.26 waves of blocks); 96^3 0.114 /
-// 0.114-0.117 ms (0.95 waves); 64^3 0.073 / 0.067 ms (0.63 waves).
-// Without a device to ask, no.
-bool fp0_split_pays(const Geom& g) {
+// The banded form's windows are placed with float coordinates, off by less
+// than its 0.05 voxels of margin up to here.
+bool fp0_band_ok(const Geom& g) {
+  constexpr int kMax = 1 << 16;
+  return g.SY <= kMax && g.SX <= kMax && g.PX <= kMax;
+}
+
+// Whether the banded 4-height form splits a run's lines over four warps: when
+// its unsplit blocks fill less than a wave.  A per call, unsplit / split:
+// 32^3 and 128 angles (64 blocks) 16.5 / 8.3 us; 64^3 and 128 (256 blocks)
+// 28.8 / 22.6; 256 x 256 x 12 and 180 (360) 173 / 121; 384 x 384 x 16 and 180
+// (540) 273 / 243; 128^3 and 192 (1536 blocks, 1.7 waves) 147 / 147; 96^3 and
+// 300 (1800) 124 / 131.  Without a device to ask, no.
+bool fp0_band_split(const Geom& g, int runs_per_warp) {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
@@ -203,16 +209,12 @@ bool fp0_split_pays(const Geom& g) {
     cudaGetLastError();
     return false;
   }
-  const double resident = 8.0 * sms;  // 4-height form: 8 blocks of 4 warps per SM
-  const double blocks = (double)ceil_div(g.PX, 4 * FP0_WARPS) *
-                        (g.n_ang < kMaxGridYZ ? g.n_ang : kMaxGridYZ) * ceil_div(g.H, 32 * 4);
-  const double w = blocks / resident;
-  if (w <= 0.0 || w >= 2.0) return false;
-  return std::ceil(2.0 * w) < 2.0 * std::ceil(w) || w <= 0.75;
+  const double blocks = (double)ceil_div(g.PX, 4 * runs_per_warp * FP0_WARPS) * g.n_ang;
+  return blocks < 6.0 * sms;  // 5 or 6 resident blocks per SM
 }
 
 Fp0Config fp0_config(const Geom& g, bool vec4, int variant) {
-  Fp0Config c{vec4 ? 4 : 1, 4, false, FP0_UNROLL, 32, false, false, 0};
+  Fp0Config c{vec4 ? 4 : 1, 4, false, FP0_UNROLL, 32, false, false, 0, 0};
   const bool dflt = variant == 0;
   if (dflt) variant = 16;  // the default
   switch (variant) {
@@ -242,12 +244,15 @@ Fp0Config fp0_config(const Geom& g, bool vec4, int variant) {
     c.R = vec4 ? 4 : 1;
     c.un = FP0_UNROLL;
     c.staged = 0;
-    // the default's 4-height form keeps neighbouring bins per block: angle
-    // groups measured slower there (128^3, 192 angles: 0.223 against
-    // 0.2095 ms); with few blocks it splits each bin run over two warps
+    // the default's 4-height form is banded, with the fewest lanes per run that
+    // hold the heights, and splits a run's lines over four warps when its
+    // blocks fill less than one wave
     if (dflt) {
       c.agroup = false;
-      c.split = vec4 && fp0_split_pays(g);
+      if (vec4 && fp0_band_ok(g)) {
+        c.band = g.H <= 16 ? 8 : g.H <= 32 ? 4 : g.H <= 64 ? 2 : 1;
+        c.split = fp0_band_split(g, c.band);
+      }
     }
   }
   return c;
@@ -258,7 +263,8 @@ Fp0Config fp0_config(const Geom& g, bool vec4, int variant) {
 // class slab's rows and columns together hold about as much, rows and
 // columns split evenly over the slabs.
 long long fp0_chunk_bytes(const Geom& g, const Fp0Config& c) {
-  const long long chunk_h = 32 * c.R > 128 ? 32 * c.R : 128;
+  long long chunk_h = 32 * c.R > 128 ? 32 * c.R : 128;
+  if (c.band && g.H < chunk_h) chunk_h = g.H;  // (the others' plans predate this)
   return (long long)g.SY * g.SX * chunk_h * 4;
 }
 
@@ -458,9 +464,12 @@ cudaError_t launch_slab_aligned(const SlabLaunch& L, cudaStream_t stream, int* l
 }
 
 cudaError_t launch_slab_config(const Fp0Config& c, const SlabLaunch& L, cudaStream_t s, int* n) {
+  if (c.band)
+    return launch_fp_band(BandLaunch{L.x, L.y, L.angles, L.g, L.slab, L.accumulate, L.a_lo, L.a_hi,
+                                     L.programmatic, L.vec_out},
+                          c.band, c.split, s, n);
   if (!L.vec_out && c.R != 1) {  // the default's forms (fp0_vec4)
     if (c.R == 8) return launch_slab<8, 4, true, 2, false, false, false>(L, s, n);
-    if (c.split) return launch_slab<4, 4, false, FP0_UNROLL, true, false, false>(L, s, n);
     return launch_slab<4, 4, false, FP0_UNROLL, false, false, false>(L, s, n);
   }
   if (c.R == 8 && c.staged) {
@@ -510,24 +519,38 @@ cudaError_t launch_fp_z0_config(const float* x, float* y, const float* angles, c
 }
 
 // The heights of a call as (first height, count) parts: one part, or with 8
-// heights per lane an 8-height part and a 4-height remainder (r8_heights).
+// heights per lane an 8-height part and 4-height parts for the rest
+// (r8_heights).  The default's banded 4-height form also takes a rest of 129 to
+// 192 heights, as 128 and what is left: about 46 + 27 clocks per SM, line and
+// run of bins against 76 for a whole 256-height chunk.
 struct HeightParts {
   int n;
-  Geom g[2];
-  int h0[2];
+  Geom g[3];
+  int h0[3];
 };
 
 HeightParts fp0_parts(const Geom& g, bool vec4, int variant) {
-  HeightParts p{1, {g, g}, {0, 0}};
-  if (fp0_config(g, vec4, variant).R == 8) {
-    const int H8 = r8_heights(g.H);
-    if (H8 < g.H) {
-      p.n = 2;
-      p.g[0].H = H8;
-      p.g[1].H = g.H - H8;
-      p.h0[1] = H8;
-    }
+  HeightParts p{0, {g, g, g}, {0, 0, 0}};
+  const auto add = [&](int h0, int H) {
+    p.h0[p.n] = h0;
+    p.g[p.n].H = H;
+    ++p.n;
+  };
+  if (fp0_config(g, vec4, variant).R != 8) {
+    add(0, g.H);
+    return p;
   }
+  int H8 = r8_heights(g.H);
+  const int full = g.H / 256 * 256, rest = g.H - full;
+  if (variant == 0 && fp0_band_ok(g) && rest > 128 && rest <= 192) {
+    H8 = full;
+    if (full > 0) add(0, full);
+    add(full, 128);
+    if (rest > 128) add(full + 128, rest - 128);
+    return p;
+  }
+  if (H8 > 0) add(0, H8);
+  if (H8 < g.H) add(H8, g.H - H8);
   return p;
 }
 
@@ -570,7 +593,7 @@ int launches_forward_z0(const float* x, const float* y, const Geom& g) {
   for (int i = 0; i < hp.n; ++i) {
     const Fp0Config c = fp0_config(hp.g[i], vec4, v);
     const long long per =
-        (c.agroup || c.staged) ? (long long)kMaxGridYZ * FP0_WARPS : kMaxGridYZ;
+        ((c.agroup && !c.band) || c.staged) ? (long long)kMaxGridYZ * FP0_WARPS : kMaxGridYZ;
     n += (int)(fp0_slabs(hp.g[i], c) * ceil_div(hp.g[i].n_ang, per));
   }
   return n;
@@ -627,10 +650,13 @@ cudaError_t launch_forward_z0_rest(const float* x, float* y, const float* angles
                                    const Geom& g, cudaStream_t stream, int* launches) {
   const bool vec4 = fp0_vec4(x, y, g);
   const HeightParts hp = fp0_parts(g, vec4, kernel_variant(OP_FORWARD_Z0));
-  if (hp.n < 2) return cudaSuccess;
-  const Fp0Config c = fp0_config(hp.g[1], vec4, kernel_variant(OP_FORWARD_Z0));
-  return launch_fp_z0_config(x + hp.h0[1], y + hp.h0[1], angles, hp.g[1], c, 0, 1 << 30,
-                             stream, launches);
+  for (int i = 1; i < hp.n; ++i) {
+    const Fp0Config c = fp0_config(hp.g[i], vec4, kernel_variant(OP_FORWARD_Z0));
+    const cudaError_t e = launch_fp_z0_config(x + hp.h0[i], y + hp.h0[i], angles, hp.g[i], c, 0,
+                                              1 << 30, stream, launches);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace vp

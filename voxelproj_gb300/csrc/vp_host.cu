@@ -625,7 +625,7 @@ cudaError_t z2_backward_chunked(const float* y_host, float* x_host, const float*
     float *in_d[2] = {}, *out_d[2] = {}, *ws[2] = {}, *as = nullptr;
     const float* ad = nullptr;
     const bool pipelined = z2_uses_transpose(gc);
-    const size_t ws_elems = z2_workspace_bytes(gc) / sizeof(float);
+    const size_t ws_elems = pipelined ? z2_workspace_bytes(gc) / sizeof(float) : 0;
     const int slots = nchunks > 1 ? 2 : 1;
     for (int i = 0; i < slots; ++i) {
       VP_TRY(buf.get(pool, (size_t)Hc * bins * sizeof(float), &in_d[i]));
@@ -683,7 +683,7 @@ cudaError_t z2_backward_chunked(const float* y_host, float* x_host, const float*
         else
           VP_TRY(cudaMemsetAsync(out_d[k & 1], 0, hc * vox * sizeof(float), t));
         VP_TRY(launch_backward_z2(in_d[k & 1], out_d[k & 1], ad, gk, t));
-        *launches += launches_z2(gk, false);
+        ++*launches;
         VP_TRY(cudaMemcpyAsync(x_host + h0 * vox, out_d[k & 1], hc * vox * sizeof(float),
                                cudaMemcpyDefault, t));
       }
@@ -826,8 +826,14 @@ cudaError_t z2_host(bool forward, const float* in_host, float* out_host, const f
                                s));
       else
         VP_TRY(cudaMemsetAsync(ys, 0, (size_t)H * bins * sizeof(float), s));
-      VP_TRY(launch_forward_thin(xs, ys, ad, gk, 2, s));
-      *launches += launches_z2(gk, true);
+      if (z2_can_transpose(gk)) {
+        VP_TRY(buf.get(pool, z2_workspace_bytes(gk), &ws));
+        VP_TRY(forward_z2_transposed(xs, ys, ad, gk, ws, s));
+        *launches += launches_z2(gk, true);
+      } else {
+        VP_TRY(launch_forward_thin(xs, ys, ad, gk, 2, s));
+        *launches += launches_forward_thin(gk);
+      }
       VP_TRY(cudaMemcpyAsync(y_host, ys, (size_t)H * bins * sizeof(float), cudaMemcpyDefault, s));
     }
     if (!g.accumulate && g.Hy > H) {

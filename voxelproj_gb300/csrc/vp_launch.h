@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include "vp_common.cuh"
+#include "vp_fp_z0.cuh"
 
 namespace vp {
 
@@ -53,6 +54,24 @@ enum Op : int { OP_FORWARD_Z0 = 0, OP_BACKWARD_Z0 = 1, OP_FORWARD_Z2 = 2, OP_BAC
                 OP_COUNT = 4 };
 int kernel_variant(int op);
 
+// The banded z_order 0 forward (vp_fp_band.cu): one slab launch on angles
+// [a_lo, a_hi); runs_per_warp (1, 2, 4, 8) runs of 4 bins share a warp (more
+// than one: H <= 128 / runs_per_warp), split spreads their lines over the 4
+// warps of a block.  x's rows are 16-byte aligned.
+struct BandLaunch {
+  const float* x;
+  float* y;
+  const float* angles;
+  Geom g;
+  detail::Slab slab;
+  int accumulate;
+  int a_lo, a_hi;
+  bool programmatic;  // follows this call's previous slab launch
+  bool vec_out;       // y's rows take float4 stores
+};
+cudaError_t launch_fp_band(const BandLaunch& L, int runs_per_warp, bool split,
+                           cudaStream_t stream, int* launches);
+
 // Few heights (vp_thin.cu): the arrays in z_order z.
 cudaError_t launch_forward_thin(const float* x, float* y, const float* angles, const Geom& g,
                                 int z, cudaStream_t stream);
@@ -65,7 +84,7 @@ int launches_forward_thin(const Geom& g);
 // scalar and 4-height kernels: A 455 -> 53 us (1 height), 573 -> 116 (4),
 // 582 -> 200 (8), but 583 -> 545 (16) and 477 -> 529 (19); A^T 363 -> 39 (1),
 // 367 -> 67 (3), 378 -> 107 (7), but 321 -> 644 (16).
-inline bool z0_forward_thin(const Geom& g) { return g.H <= 8; }
+inline bool z0_forward_thin(const Geom& g) { return g.H <= 4; }
 inline bool z0_backward_thin(const Geom& g) { return g.H <= 7 && g.H % 4 != 0; }
 
 // dst rows of Hd floats from src rows of Hs: heights [0, H), then zeros; dst
@@ -74,9 +93,14 @@ cudaError_t pad_heights(const float* src, float* dst, long long rows, int Hs, in
                         cudaStream_t stream);
 
 // z_order 2 through the z_order 0 kernels (vp_z2.cu).
+// From 32 heights on always; from 5 on the forward does where it has the
+// workspace (z2_workspace_bytes, more than 0 then), else it runs the kernel
+// for few heights, which needs none: 384 x 384 x 16, 180 angles 685 against
+// 262 us with the transposes, 512 x 512 x 4 and 360 662 against 780 us.
 bool z2_uses_transpose(const Geom& g);
+bool z2_can_transpose(const Geom& g);
 size_t z2_workspace_bytes(const Geom& g);
-int launches_z2(const Geom& g, bool forward);
+int launches_z2(const Geom& g, bool forward);  // of the transposed form
 cudaError_t forward_z2_transposed(const float* x, float* y, const float* angles, const Geom& g,
                                   float* ws, cudaStream_t stream);
 cudaError_t backward_z2_transposed(const float* y, float* x, const float* angles, const Geom& g,

@@ -29,7 +29,8 @@ constexpr int TT = 32;         // tile edge
 constexpr int TROWS = 8;       // thread rows per tile (each thread moves TT/TROWS elements)
 constexpr int KE = TT / TROWS;
 
-// dst[c * dst_ld + r] (+)= src[r * src_ld + c] for r < rows, c < cols.
+// dst[c * dst_ld + r] (+)= src[r * src_ld + c] for r < rows, c < cols; the
+// storing form writes zeros for rows <= r < rows_out (pad heights).
 // Tiles are visited with a grid-stride loop so any matrix fits one launch.
 // ADD: add into dst.  The adding form moves two neighbouring tiles per
 // iteration and issues every load of them (the source rows into shared
@@ -41,11 +42,11 @@ constexpr int KE = TT / TROWS;
 template <bool ADD>
 __global__ void __launch_bounds__(TT * TROWS)
     transpose_kernel(const float* __restrict__ src, float* __restrict__ dst, long long rows,
-                     long long cols, long long src_ld, long long dst_ld) {
+                     long long cols, long long src_ld, long long dst_ld, long long rows_out) {
   constexpr int TPI = ADD ? 2 : 1;  // tiles per iteration
   __shared__ float tile[TPI][TT][TT + 1];
   const long long tiles_c = (cols + TT - 1) / TT;
-  const long long tiles_r = (rows + TT - 1) / TT;
+  const long long tiles_r = (rows_out + TT - 1) / TT;
   const long long ntiles = tiles_c * tiles_r;
   const int tx = threadIdx.x, ty = threadIdx.y;
   for (long long t0 = (long long)blockIdx.x * TPI; t0 < ntiles;
@@ -62,7 +63,8 @@ __global__ void __launch_bounds__(TT * TROWS)
       for (int k = 0; k < KE; ++k) {
         const long long r = r0 + ty + k * TROWS;
         const long long c = c0 + tx;
-        if (tv && r < rows && c < cols) tile[j][ty + k * TROWS][tx] = __ldg(src + r * src_ld + c);
+        if (tv && r < rows_out && c < cols)
+          tile[j][ty + k * TROWS][tx] = ADD || r < rows ? __ldg(src + r * src_ld + c) : 0.0f;
       }
 #pragma unroll
       for (int k = 0; k < KE; ++k) {
@@ -82,7 +84,7 @@ __global__ void __launch_bounds__(TT * TROWS)
       for (int k = 0; k < KE; ++k) {
         const long long c = c0 + ty + k * TROWS;
         const long long r = r0 + tx;
-        if (tv && r < rows && c < cols) {
+        if (tv && r < rows_out && c < cols) {
           const float v = tile[j][tx][ty + k * TROWS];
           if constexpr (ADD) dst[c * dst_ld + r] = old[j][k] + v;
           else dst[c * dst_ld + r] = v;
@@ -94,9 +96,11 @@ __global__ void __launch_bounds__(TT * TROWS)
 }
 
 cudaError_t transpose(const float* src, float* dst, long long rows, long long cols,
-                      long long src_ld, long long dst_ld, int accumulate, cudaStream_t stream) {
+                      long long src_ld, long long dst_ld, int accumulate, cudaStream_t stream,
+                      long long pad_to = 0) {
   if (rows <= 0 || cols <= 0) return cudaSuccess;
-  const long long ntiles = ((rows + TT - 1) / TT) * ((cols + TT - 1) / TT);
+  const long long rows_out = rows < pad_to ? pad_to : rows;
+  const long long ntiles = ((rows_out + TT - 1) / TT) * ((cols + TT - 1) / TT);
   const long long iters = accumulate ? (ntiles + 1) / 2 : ntiles;
   // one resident wave of blocks (the tiles are dealt out by block index)
   int dev = 0, sms = 152, per_sm = 0;
@@ -111,10 +115,10 @@ cudaError_t transpose(const float* src, float* dst, long long rows, long long co
   const unsigned grid = (unsigned)(iters < cap ? iters : cap);
   if (accumulate)
     transpose_kernel<true><<<grid, dim3(TT, TROWS), 0, stream>>>(src, dst, rows, cols, src_ld,
-                                                                 dst_ld);
+                                                                 dst_ld, rows);
   else
     transpose_kernel<false><<<grid, dim3(TT, TROWS), 0, stream>>>(src, dst, rows, cols, src_ld,
-                                                                  dst_ld);
+                                                                  dst_ld, rows_out);
   return cudaGetLastError();
 }
 
@@ -154,14 +158,15 @@ cudaError_t pad_heights(const float* src, float* dst, long long rows, int Hs, in
 
 bool z2_uses_transpose(const Geom& g) { return g.H >= 32; }
 
+bool z2_can_transpose(const Geom& g) { return g.H >= 5; }
+
 size_t z2_workspace_bytes(const Geom& g) {
-  if (!z2_uses_transpose(g)) return 0;
+  if (!z2_can_transpose(g)) return 0;
   const long long Hp = round4(g.H);
   return (size_t)(((long long)g.SY * g.SX + (long long)g.n_ang * g.PX) * Hp) * sizeof(float);
 }
 
 int launches_z2(const Geom& g, bool forward) {
-  if (!z2_uses_transpose(g)) return forward ? launches_forward_thin(g) : 1;
   // the transposed path runs the z_order 0 kernels on 16-byte aligned scratch
   // with a height extent that is a multiple of 4
   Geom g0 = g;
@@ -186,11 +191,11 @@ cudaError_t z2_project(bool forward, const float* in, const float* angles, const
   g0.H = g0.Hx = g0.Hy = (int)Hp;
   g0.accumulate = 0;
   if (forward) {
-    const cudaError_t e = transpose(in, xt, g.H, nvox, nvox, Hp, 0, stream);
+    const cudaError_t e = transpose(in, xt, g.H, nvox, nvox, Hp, 0, stream, Hp);
     if (e != cudaSuccess) return e;
     return launch_forward_z0(xt, yt, angles, g0, stream);
   }
-  const cudaError_t e = transpose(in, yt, g.H, nbin, nbin, Hp, 0, stream);
+  const cudaError_t e = transpose(in, yt, g.H, nbin, nbin, Hp, 0, stream, Hp);
   if (e != cudaSuccess) return e;
   return launch_backward_z0(yt, xt, angles, g0, stream);
 }
@@ -213,7 +218,7 @@ cudaError_t z2_transpose_in_rows(const float* x, const Geom& g, float* ws, int l
   const long long Hp = round4(g.H);
   const long long nvox = (long long)g.SY * g.SX;
   return transpose(x + (long long)lo * g.SX, ws + (long long)lo * g.SX * Hp, g.H,
-                   (long long)(hi - lo) * g.SX, nvox, Hp, 0, stream);
+                   (long long)(hi - lo) * g.SX, nvox, Hp, 0, stream, Hp);
 }
 
 // Angles [a0, a1) of a heights-slowest sinogram in (g.H, n_ang, PX) into the
@@ -224,7 +229,7 @@ cudaError_t z2_transpose_in_angles(const float* y, const Geom& g, float* ws, int
   const long long nvox = (long long)g.SY * g.SX;
   const long long nbin = (long long)g.n_ang * g.PX;
   return transpose(y + (long long)a0 * g.PX, ws + nvox * Hp + (long long)a0 * g.PX * Hp, g.H,
-                   (long long)(a1 - a0) * g.PX, nbin, Hp, 0, stream);
+                   (long long)(a1 - a0) * g.PX, nbin, Hp, 0, stream, Hp);
 }
 
 // Angles [a0, a1) of the forward's yt (n_ang, PX, Hp) in ws into a
