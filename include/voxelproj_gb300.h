@@ -162,6 +162,16 @@ VP_API int vp_backward_z2_ws(const float* y, int64_t y0, int64_t y1, int64_t y2,
                              const float* angles, int64_t n_angles, int flags,
                              void* workspace, size_t workspace_bytes, void* stream);
 
+/* out = A in (op VP_OP_FORWARD) or out = A^T in (VP_OP_BACKWARD) in z_order 0
+ * or 2: for outputs that the call makes, which then need no zeros written
+ * first and read back.  Every element of out is written (0 where the operator
+ * reaches none).  dims as in the calls above, input first; workspace as in
+ * vp_forward_z2_ws (may be NULL; unused in z_order 0). */
+VP_API int vp_project_store(int op, int z_order, const float* in, const int64_t in_dims[3],
+                            float* out, const int64_t out_dims[3], const float* angles,
+                            int64_t n_angles, int flags, void* workspace,
+                            size_t workspace_bytes, void* stream);
+
 /* y += A x, z_order 2, allocating nothing: for callers that may not allocate
  * device memory while they run (code that fixes its memory at start-up,
  * hosts whose own allocator owns the device).  Same arguments and results as

@@ -17,6 +17,7 @@ current torch CUDA stream of ``in``'s device and is not synchronised.
 
 from __future__ import annotations
 
+import ctypes
 import os
 
 import torch
@@ -68,29 +69,70 @@ def _check_other(t, name: str, device: torch.device, ndim: int | None) -> None:
         raise RuntimeError(f"{name} must be {ndim}D")
 
 
+try:  # the stream handle alone; the public call builds a Stream object first
+    _raw_stream = torch._C._cuda_getCurrentRawStream
+except AttributeError:  # pragma: no cover
+    def _raw_stream(index: int) -> int:
+        return torch.cuda.current_stream(index).cuda_stream
+
+
+def _z2_workspace(inp, out, forward: bool):
+    """Scratch for the transposed path from torch's caching allocator, or None."""
+    x, y = (inp, out) if forward else (out, inp)
+    nbytes = _lib.LIB.vp_z2_workspace_bytes(*x.shape, *y.shape)
+    if not nbytes:
+        return None, 0
+    return torch.empty((nbytes + 3) // 4, dtype=torch.float32, device=inp.device), nbytes
+
+
+def _on_device(device, fn):
+    """fn(stream handle) with the device current."""
+    if torch.cuda.current_device() == device.index:
+        return fn(_raw_stream(device.index))
+    with torch.cuda.device(device):
+        return fn(_raw_stream(device.index))
+
+
 def _call(fn_name: str, inp, out, angles) -> None:
     _check_in(inp)
     _check_other(out, "out", inp.device, 3)
     _check_other(angles, "angles", inp.device, None)
     if out.data_ptr() == inp.data_ptr() and inp.numel() > 0:
         raise RuntimeError("in and out must not alias")
-    with torch.cuda.device(inp.device):
-        stream = torch.cuda.current_stream(inp.device).cuda_stream
-        if fn_name.endswith("z2"):
-            # scratch for the transposed path, from torch's caching allocator
-            x, y = (inp, out) if fn_name.startswith("vp_forward") else (out, inp)
-            nbytes = _lib.LIB.vp_z2_workspace_bytes(*x.shape, *y.shape)
-            ws = torch.empty((nbytes + 3) // 4, dtype=torch.float32, device=inp.device) \
-                if nbytes else None
-            fn = getattr(_lib.LIB, fn_name + "_ws")
-            status = fn(inp.data_ptr(), *inp.shape, out.data_ptr(), *out.shape,
-                        angles.data_ptr(), angles.numel(), _flags,
-                        ws.data_ptr() if ws is not None else None, nbytes, stream)
-        else:
-            fn = getattr(_lib.LIB, fn_name)
-            status = fn(inp.data_ptr(), *inp.shape, out.data_ptr(), *out.shape,
-                        angles.data_ptr(), angles.numel(), _flags, stream)
-    _lib.check(status, fn_name[3:])
+
+    def run(stream):
+        args = (inp.data_ptr(), *inp.shape, out.data_ptr(), *out.shape, angles.data_ptr(),
+                angles.numel(), _flags)
+        if not fn_name.endswith("z2"):
+            return getattr(_lib.LIB, fn_name)(*args, stream)
+        ws, nbytes = _z2_workspace(inp, out, fn_name.startswith("vp_forward"))
+        return getattr(_lib.LIB, fn_name + "_ws")(*args, ws.data_ptr() if ws is not None else None,
+                                                  nbytes, stream)
+
+    _lib.check(_on_device(inp.device, run), fn_name[3:])
+
+
+_DIMS = ctypes.c_int64 * 3
+
+
+def project_store(forward: bool, z_order: int, inp, out, angles):
+    """out = A inp (forward) or A^T inp, whatever out held: for outputs made by the
+    call, which then need no zeros first.  Returns out."""
+    _check_in(inp)
+    _check_other(out, "out", inp.device, 3)
+    _check_other(angles, "angles", inp.device, None)
+    if out.data_ptr() == inp.data_ptr() and inp.numel() > 0:
+        raise RuntimeError("in and out must not alias")
+
+    def run(stream):
+        ws, nbytes = _z2_workspace(inp, out, forward) if z_order == 2 else (None, 0)
+        return _lib.LIB.vp_project_store(
+            _lib.VP_OP_FORWARD if forward else _lib.VP_OP_BACKWARD, z_order, inp.data_ptr(),
+            _DIMS(*inp.shape), out.data_ptr(), _DIMS(*out.shape), angles.data_ptr(),
+            angles.numel(), _flags, ws.data_ptr() if ws is not None else None, nbytes, stream)
+
+    _lib.check(_on_device(inp.device, run), ("forward_z%d" if forward else "backward_z%d") % z_order)
+    return out
 
 
 def forward_z0(inp, out, angles, block_size=(8, 8, 8)) -> None:

@@ -69,6 +69,7 @@ SIGNATURES = {
                               ctypes.c_size_t, _P]),
     "vp_backward_z2_ws": (_I, [_P, _I64, _I64, _I64, _P, _I64, _I64, _I64, _P, _I64, _I, _P,
                                ctypes.c_size_t, _P]),
+    "vp_project_store": (_I, [_I, _I, _P, _P, _P, _P, _P, _I64, _I, _P, ctypes.c_size_t, _P]),
     "vp_forward_z2_noalloc": (_I, [_P, _I64, _I64, _I64, _P, _I64, _I64, _I64, _P, _I64, _I,
                                    _P]),
     "vp_batch_create": (_I, [_P, _I, _P]),

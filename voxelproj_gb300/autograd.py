@@ -22,8 +22,7 @@ import torch
 
 from . import _CU
 
-_FWD = {0: _CU.forward_z0, 2: _CU.forward_z2}
-_BWD = {0: _CU.backward_z0, 2: _CU.backward_z2}
+_Z_ORDERS = (0, 2)
 
 
 def _angles_tensor(angles, device) -> torch.Tensor:
@@ -46,17 +45,15 @@ def _x_shape(sino_shape, vol_yx, z_order):
 
 
 def _apply_forward(x32, a32, px, z_order):
-    y = torch.zeros(_y_shape(x32.shape, a32.numel(), px, z_order), dtype=torch.float32,
+    y = torch.empty(_y_shape(x32.shape, a32.numel(), px, z_order), dtype=torch.float32,
                     device=x32.device)
-    _FWD[z_order](x32, y, a32)
-    return y
+    return _CU.project_store(True, z_order, x32, y, a32)
 
 
 def _apply_backward(y32, a32, vol_yx, z_order):
-    x = torch.zeros(_x_shape(y32.shape, vol_yx, z_order), dtype=torch.float32,
+    x = torch.empty(_x_shape(y32.shape, vol_yx, z_order), dtype=torch.float32,
                     device=y32.device)
-    _BWD[z_order](y32, x, a32)
-    return x
+    return _CU.project_store(False, z_order, y32, x, a32)
 
 
 def _vol_yx(x_shape, z_order):
@@ -68,7 +65,7 @@ class ProjectFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, angles, detector_width, z_order):
-        if z_order not in _FWD:
+        if z_order not in _Z_ORDERS:
             raise KeyError(z_order)
         a32 = _angles_tensor(angles, x.device)
         vol_yx = _vol_yx(x.shape, z_order)
@@ -91,7 +88,7 @@ class BackprojectFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, y, angles, volume_yx, z_order):
-        if z_order not in _BWD:
+        if z_order not in _Z_ORDERS:
             raise KeyError(z_order)
         a32 = _angles_tensor(angles, y.device)
         px = y.shape[1] if z_order == 0 else y.shape[2]

@@ -468,6 +468,38 @@ int vp_backward(const float* y, const int64_t y_dims[3], float* x, const int64_t
 
 }  // extern "C"
 
+extern "C" int vp_project_store(int op, int z_order, const float* in, const int64_t in_dims[3],
+                                float* out, const int64_t out_dims[3], const float* angles,
+                                int64_t n_angles, int flags, void* workspace,
+                                size_t workspace_bytes, void* stream) {
+  if (in_dims == nullptr || out_dims == nullptr) return VP_ERR_NULL_POINTER;
+  if (z_order != 0 && z_order != 2) return VP_ERR_BAD_Z_ORDER;
+  if (op != VP_OP_FORWARD && op != VP_OP_BACKWARD) return VP_ERR_BAD_FLAGS;
+  const bool fwd = op == VP_OP_FORWARD;
+  const int64_t* xd = fwd ? in_dims : out_dims;
+  const int64_t* yd = fwd ? out_dims : in_dims;
+  const float* x = fwd ? in : out;
+  const float* y = fwd ? out : in;
+  vp::Geom g;
+  bool empty = false;
+  const int s = z_order == 0
+                    ? make_geom(x, xd[0], xd[1], xd[2], y, yd[0], yd[1], yd[2], angles, n_angles,
+                                flags, &g, &empty)
+                    : make_geom(x, xd[1], xd[2], xd[0], y, yd[1], yd[2], yd[0], angles, n_angles,
+                                flags, &g, &empty);
+  if (s) return s;
+  const cudaStream_t st = (cudaStream_t)stream;
+  g.accumulate = 0;
+  if (empty || (fwd ? g.Hy : g.Hx) > g.H) {  // elements that the projection does not reach
+    const size_t n = (size_t)out_dims[0] * out_dims[1] * out_dims[2];
+    const cudaError_t e = n ? cudaMemsetAsync(out, 0, n * sizeof(float), st) : cudaSuccess;
+    if (empty || e != cudaSuccess) return finish(e, 0);
+    g.accumulate = 1;
+  }
+  return z_order == 0 ? run_z0(fwd, in, out, angles, g, st)
+                      : run_z2(fwd, in, out, angles, g, workspace, workspace_bytes, st);
+}
+
 // ---------------------------------------------------------------------------
 // Forward projection in z_order 2 without any device allocation.
 //

@@ -253,20 +253,20 @@ cudaError_t z2_transpose_out_rows(float* x, const Geom& g, const float* ws, int 
                    (long long)(hi - lo) * g.SX, g.H, Hp, nvox, add, stream);
 }
 
-// x (Hx, SY, SX) -> xt (SY, SX, Hp); yt = A xt; y (Hy, n, PX) += yt^T.
+// x (Hx, SY, SX) -> xt (SY, SX, Hp); yt = A xt; y (Hy, n, PX) (+)= yt^T.
 cudaError_t forward_z2_transposed(const float* x, float* y, const float* angles, const Geom& g,
                                   float* ws, cudaStream_t stream) {
   const cudaError_t e = z2_project(true, x, angles, g, ws, stream);
   if (e != cudaSuccess) return e;
-  return z2_transpose_out(true, y, g, ws, 1, stream);
+  return z2_transpose_out(true, y, g, ws, g.accumulate, stream);
 }
 
-// y (Hy, n, PX) -> yt (n, PX, Hp); xt = A^T yt; x (Hx, SY, SX) += xt^T.
+// y (Hy, n, PX) -> yt (n, PX, Hp); xt = A^T yt; x (Hx, SY, SX) (+)= xt^T.
 cudaError_t backward_z2_transposed(const float* y, float* x, const float* angles, const Geom& g,
                                    float* ws, cudaStream_t stream) {
   const cudaError_t e = z2_project(false, y, angles, g, ws, stream);
   if (e != cudaSuccess) return e;
-  return z2_transpose_out(false, x, g, ws, 1, stream);
+  return z2_transpose_out(false, x, g, ws, g.accumulate, stream);
 }
 
 }  // namespace vp

@@ -93,18 +93,14 @@ class Operator:
         n = self.a.numel()
         self.sino_shape = ((n, self.px, self.vol_shape[2]) if z_order == 0
                            else (self.vol_shape[0], n, self.px))
-        self._fwd = _CU.forward_z0 if z_order == 0 else _CU.forward_z2
-        self._bwd = _CU.backward_z0 if z_order == 0 else _CU.backward_z2
 
     def A(self, x, out=None):
-        out = torch.zeros(self.sino_shape, device=x.device) if out is None else out.zero_()
-        self._fwd(x, out, self.a)
-        return out
+        out = torch.empty(self.sino_shape, device=x.device) if out is None else out
+        return _CU.project_store(True, self.z, x, out, self.a)
 
     def AT(self, y, out=None):
-        out = torch.zeros(self.vol_shape, device=y.device) if out is None else out.zero_()
-        self._bwd(y, out, self.a)
-        return out
+        out = torch.empty(self.vol_shape, device=y.device) if out is None else out
+        return _CU.project_store(False, self.z, y, out, self.a)
 
 
 def sirt(op: Operator, b: torch.Tensor, iters: int, x0: torch.Tensor | None = None):

@@ -102,7 +102,7 @@ def _input_gpu(v) -> torch.Tensor:
 def _finish(out, out_gpu, work, src_kind, src_device):
     """Copies back into a caller's container or returns a new array in the
     input's kind (wrappers.py:57-73)."""
-    if work is not out_gpu:
+    if work is not None and work is not out_gpu:
         out_gpu.copy_(work)
     if isinstance(out, np.ndarray):
         if out.dtype == np.float32 and out.flags.c_contiguous and out.flags.writeable:
@@ -204,6 +204,9 @@ def forward(x, angles, y, z_order=0, block_size=[8, 8, 8]):
         return _host_call("vp_forward_z%d_host" % z_order, x, y, angles, shape, kind)
     x_gpu = _input_gpu(x)
     a_gpu = _angles_gpu(angles, x_gpu.device)
+    if y is None or isinstance(y, tuple):
+        out = torch.empty(shape if y is None else y, dtype=torch.float32, device=x_gpu.device)
+        return _finish(None, _CU.project_store(True, z_order, x_gpu, out, a_gpu), None, kind, device)
     y_gpu = gpu_array_with_default_shape(y, shape=shape)
     work = y_gpu if y_gpu.is_contiguous() else y_gpu.contiguous()
     fn(x_gpu, work, a_gpu, block_size=block_size)
@@ -224,6 +227,10 @@ def backward(y, angles, x, z_order=0, block_size=[8, 8, 8]):
         return _host_call("vp_backward_z%d_host" % z_order, y, x, angles, shape, kind)
     y_gpu = _input_gpu(y)
     a_gpu = _angles_gpu(angles, y_gpu.device)
+    if x is None or isinstance(x, tuple):
+        out = torch.empty(shape if x is None else x, dtype=torch.float32, device=y_gpu.device)
+        return _finish(None, _CU.project_store(False, z_order, y_gpu, out, a_gpu), None, kind,
+                       device)
     x_gpu = gpu_array_with_default_shape(x, shape=shape)
     work = x_gpu if x_gpu.is_contiguous() else x_gpu.contiguous()
     fn(y_gpu, work, a_gpu, block_size=block_size)
