@@ -111,11 +111,11 @@ __device__ __forceinline__ float bin_centre(float q, int i, float cent_major, fl
 struct ThinChunk {
   int i0, nl, m0, nh;  // lines [i0, i0 + nl), the tile's first voxel, heights
   float cent_major, cent_minor, sh_major, inv;
-  bool four;           // 4 voxels per bin and line, else 3
 };
 
-// This lane's bin on the lines of one chunk.
-template <int RH, int LC, int TRIG, bool MX>
+// This lane's bin on the lines of one chunk.  FOUR: 4 voxels per bin and line,
+// else 3.
+template <int RH, int LC, int TRIG, bool MX, bool FOUR>
 __device__ __forceinline__ void gather_lines(float (&acc)[RH],
                                              const float (*tl)[LC][ThinTile<LC>::W],
                                              const ThinChunk& c, float fp, const AngleConst& k,
@@ -124,14 +124,13 @@ __device__ __forceinline__ void gather_lines(float (&acc)[RH],
   for (int l = 0; l < c.nl; ++l) {
     const int i = c.i0 + l;
     const float u = bin_centre(fp, i, c.cent_major, c.sh_major, c.inv, c.cent_minor, pcent);
-    const int first = (c.four ? (int)floorf(u) : __float2int_rn(u)) - 1;
-    // (inside the tile but for rounding)
-    const int o = max(0, min(first - c.m0, ThinTile<LC>::W - 4));
+    const int first = (FOUR ? (int)floorf(u) : __float2int_rn(u)) - 1;
+    // (inside the tile but for rounding; one unsigned minimum bounds both sides)
+    const int o = (int)min((unsigned)(first - c.m0), (unsigned)(ThinTile<LC>::W - 4));
     const float rel_major = (float)i - c.cent_major;
     const float rel_first = (float)(c.m0 + o) - c.cent_minor;
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      if (t == 3 && !c.four) break;
+    for (int t = 0; t < (FOUR ? 4 : 3); ++t) {
       const float d = fabsf(bin_distance<MX, TRIG>(fp, rel_first + (float)t, rel_major, k, pcent));
       const float z = 0.5f - d;
       const float e = __saturatef((k.b - 0.5f) - d);
@@ -210,9 +209,14 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
         tile_load<RH, LC, UT, false>(tl, corner, l, m, nm, l < nl, nh, st.xh, s_maj, s_min, m0, n_minor);
     }
     __syncwarp();
-    const ThinChunk c{i0, nl, m0, nh, cent_major, cent_minor, sh_major, inv, four};
-    if (minor_x) gather_lines<RH, LC, TRIG, true>(acc, tl, c, fp, k, g.pcent);
-    else gather_lines<RH, LC, TRIG, false>(acc, tl, c, fp, k, g.pcent);
+    const ThinChunk c{i0, nl, m0, nh, cent_major, cent_minor, sh_major, inv};
+    if (minor_x) {
+      if (four) gather_lines<RH, LC, TRIG, true, true>(acc, tl, c, fp, k, g.pcent);
+      else gather_lines<RH, LC, TRIG, true, false>(acc, tl, c, fp, k, g.pcent);
+    } else {
+      if (four) gather_lines<RH, LC, TRIG, false, true>(acc, tl, c, fp, k, g.pcent);
+      else gather_lines<RH, LC, TRIG, false, false>(acc, tl, c, fp, k, g.pcent);
+    }
   }
 
   // the block's four sums
