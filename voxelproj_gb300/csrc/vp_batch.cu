@@ -50,6 +50,7 @@
 #include "vp_bp_block.cuh"
 #include "vp_bp_runs.cuh"
 #include "vp_common.cuh"
+#include "vp_fp_band.cuh"
 #include "vp_fp_z0.cuh"
 #include "vp_launch.h"
 
@@ -90,6 +91,10 @@ struct BatchDesc {
   // agroup, a group of 4 neighbouring angles (one per warp, on the same
   // 4-bin run); units: item columns per row
   int cls, wy, wx, units, agroup, rows;
+  // forward with 4 heights per lane: runs per warp of the banded form
+  // (vp_fp_band.cuh), 0 = candidate lists; an item column is then one set of
+  // runs (agroup) or one per warp
+  int band;
   // run adjoint: runs and run groups of each class
   int nruns0, groups0, nruns1, groups1;
   // block adjoint: blocks along x, blocks, block groups
@@ -100,8 +105,9 @@ struct BatchDesc {
 // lists (as the single-problem forward, leaving the rest of the SM's unified
 // storage to L1); the adjoint bodies their run tables, or the 2x2 block
 // tables where the 4-height adjoint carries that variant too.
-struct FwdSmem {
+union FwdSmem {
   float4 cand[BATCH_WARPS][Fp0Cap<4>::list];
+  BandSmem band[BATCH_WARPS];
 };
 struct RunsSmem {
   RunEntry tab[BATCH_WARPS][BPR_CHUNK];
@@ -195,6 +201,27 @@ __device__ __noinline__ void run_fwd_item(const BatchDesc& d, int stage, int in_
   signal_done(slot->counter);
 }
 
+// The same with the banded form, G runs per warp.
+template <int G>
+__device__ __noinline__ void run_fwd_band_item(const BatchDesc& d, int stage, int in_stage, int hc,
+                                               FwdSmem& sm, WaitSlot* slot, int w, int lane,
+                                               unsigned* counters, int* error,
+                                               const WaitLimits& lim) {
+  const int row = in_stage / d.units;
+  const int u = in_stage - row * d.units;
+  const Slab slab = slab_of(stage, d.cls, d.wy, d.wx, d.g.SY, d.g.SX);
+  if (lane == 0)
+    *slot = WaitSlot{counters + d.counter_base + ((size_t)hc * d.rows + row) * d.units + u,
+                     error, stage > 0 ? (unsigned)(stage * BATCH_WARPS) + lim.extra : 0u,
+                     lim.spins};
+  __syncwarp();
+  const int a = d.agroup ? row * BATCH_WARPS + w : row;
+  const int set = d.agroup ? u : u * BATCH_WARPS + w;
+  const int h = G > 1 ? (lane % (32 / G)) * 4 : hc * 128 + lane * 4;
+  fp_band_warp<G>(d.in, d.out, d.angles, d.g, set * G, a, h, slab, &sm.band[w], SlotWait{slot});
+  signal_done(slot->counter);
+}
+
 // A class-0 item (group grp) is the 4 x 4 voxel tile of band grp / nmaj
 // (rows 4 * band ..) and columns 4 * (grp % nmaj) .., one row per warp
 // (run_origin<0>); its counter counts its warps done.  A class-1 run (column
@@ -260,12 +287,11 @@ __host__ __device__ inline int body_of(const BatchDesc& d) {
 // Resident blocks per SM the registers must allow, so that each body keeps
 // its single-problem kernel's occupancy despite the item bookkeeping:
 // 8-height forwards 7 (72 registers, a few spilled; at 6 blocks the 64-cube
-// batch took 332 ms instead of 322), 4-height forward 8 (64, as the
-// single-problem 4-height kernel; at 7 blocks and 72 registers it ran 1.7%
-// slower than its single calls), 8-height run adjoints 5 (96); the 4-height
+// batch took 332 ms instead of 322), 4-height forward 6 (80, as the banded
+// single-problem kernel), 8-height run adjoints 5 (96); the 4-height
 // adjoints as the compiler chooses (72).
 constexpr int batch_min_blocks(int body) {
-  return body == B_FWD4 ? 8 : (body == B_FWD8 || body == B_FWD8F) ? 7
+  return body == B_FWD4 ? 6 : (body == B_FWD8 || body == B_FWD8F) ? 7
          : (body == B_BWD8 || body == B_BWD8F)                  ? 5
                                                                 : 0;
 }
@@ -347,8 +373,15 @@ __global__ void __launch_bounds__(BATCH_THREADS, batch_min_blocks(BODY))
       constexpr int R = BODY == B_FWD4 ? 4 : 8;
       const int per_stage = d.rows * d.units;
       const int stage = in_chunk / per_stage;
-      run_fwd_item<R, BODY == B_FWD8F>(d, stage, in_chunk - stage * per_stage, hc, sm,
-                                       &slots[w], w, lane, counters, error, lim);
+      const int in_stage = in_chunk - stage * per_stage;
+      const auto item_of = [&](auto run) {
+        run(d, stage, in_stage, hc, sm, &slots[w], w, lane, counters, error, lim);
+      };
+      if (BODY != B_FWD4 || d.band == 0) item_of(run_fwd_item<R, BODY == B_FWD8F>);
+      else if (d.band == 1) item_of(run_fwd_band_item<1>);
+      else if (d.band == 2) item_of(run_fwd_band_item<2>);
+      else if (d.band == 4) item_of(run_fwd_band_item<4>);
+      else item_of(run_fwd_band_item<8>);
     } else {
       // the adjoint bodies run faster on a register copy of the descriptor
       // (108.3 against 110.6 ms on the 64-cube workload)
@@ -427,8 +460,11 @@ namespace {
 
 // Work items of one height part: heights [0, g.H) of in / out, R heights
 // per lane for the runs adjoint (the forward takes R from its plan).
+// planH: the heights whose forward slab plan the part follows (a part of a
+// problem planned with 8 heights per lane keeps that plan, and so its sums, when
+// it runs with 4).
 int part_desc(const vp_batch_problem& p, const vp::Geom& g, const float* in, float* out, int R,
-              vp::BatchDesc* d) {
+              vp::BatchDesc* d, int planH = 0) {
   std::memset(d, 0, sizeof(*d));
   d->g = g;
   d->in = in;
@@ -437,8 +473,14 @@ int part_desc(const vp_batch_problem& p, const vp::Geom& g, const float* in, flo
   if (p.op == VP_OP_FORWARD) {
     // the single-problem forward's plan for this variant (0: the batch's
     // default, kBatchForwardDefault)
-    const vp::Fp0Plan pl =
-        vp::forward_z0_plan(g, true, p.variant ? p.variant : vp::kBatchForwardDefault);
+    vp::Geom gp = g;
+    if (planH > 0) gp.H = planH;
+    vp::Fp0Plan pl =
+        vp::forward_z0_plan(gp, true, p.variant ? p.variant : vp::kBatchForwardDefault);
+    if (planH > 0) {
+      pl.R = 4;
+      pl.un = vp::detail::FP0_UNROLL;
+    }
     if (pl.KW != 4 || pl.split || pl.staged ||
         (pl.R == 8 ? pl.un != 2 : pl.un != vp::detail::FP0_UNROLL))
       return VP_ERR_BATCH;  // bodies the batch does not carry
@@ -449,8 +491,16 @@ int part_desc(const vp_batch_problem& p, const vp::Geom& g, const float* in, flo
     d->wx = pl.wx;
     d->nstages = pl.nslabs;
     d->agroup = pl.agroup ? 1 : 0;
+    // the default's 4-height parts are banded; their warps take neighbouring run
+    // sets, or, where an angle has fewer than 8 sets, neighbouring angles
+    int G = 1;
+    if (p.variant == 0 && pl.R == 4 && vp::fp0_band_ok(g)) {
+      d->band = G = vp::fp0_band_runs(g.H);
+      pl.agroup = vp::ceil_div_u(g.PX, 4ll * G) < 8;
+      d->agroup = pl.agroup ? 1 : 0;
+    }
     d->rows = pl.agroup ? (int)vp::ceil_div_u(g.n_ang, vp::BATCH_WARPS) : g.n_ang;
-    d->units = (int)vp::ceil_div_u(g.PX, pl.agroup ? 4ll : 4ll * vp::BATCH_WARPS);
+    d->units = (int)vp::ceil_div_u(g.PX, pl.agroup ? 4ll * G : 4ll * G * vp::BATCH_WARPS);
     d->per_chunk = (long long)d->nstages * d->rows * d->units;
   } else if (p.variant == 0 || p.variant == 6 || p.variant == 7) {
     d->kind = vp::K_BWD_RUNS;
@@ -527,18 +577,25 @@ int batch_desc(const vp_batch_problem& p, std::vector<vp::BatchDesc>* out) {
   else if ((p.variant == 0 || p.variant == 7) && H > 128)
     R = 8;
   const int H8 = R == 8 ? vp::r8_heights(g.H) : g.H;
-  vp::BatchDesc d;
-  vp::Geom g0 = g;
-  g0.H = H8;
-  if (int st = part_desc(p, g0, p.in, p.out, R, &d)) return st;
-  out->push_back(d);
-  if (H8 < g.H) {
-    vp::Geom g1 = g;
-    g1.H = g.H - H8;
-    if (int st = part_desc(p, g1, p.in + H8, p.out + H8, 4, &d)) return st;
-    out->push_back(d);
+  const auto add = [&](int h0, int n, int planH) {
+    vp::Geom gp = g;
+    gp.H = n;
+    vp::BatchDesc d;
+    const int st = part_desc(p, gp, p.in + h0, p.out + h0, h0 < H8 ? R : 4, &d, planH);
+    if (st == VP_OK) out->push_back(d);
+    return st;
+  };
+  // the default's forward takes a last chunk of 129 to 192 heights by banded
+  // 4-height parts, as the single-problem default does (fp0_parts)
+  const int full = H8 / 256 * 256, rest = H8 - full;
+  if (fwd && p.variant == 0 && R == 8 && rest > 128 && rest <= 192 && vp::fp0_band_ok(g)) {
+    if (full > 0)
+      if (int st = add(0, full, 0)) return st;
+    if (int st = add(full, 128, H8)) return st;
+    return add(full + 128, rest - 128, H8);
   }
-  return VP_OK;
+  if (int st = add(0, H8, 0)) return st;
+  return H8 < g.H ? add(H8, g.H - H8, 0) : VP_OK;
 }
 
 // A plan's descriptors and bookkeeping for a set of problems: descriptors

@@ -188,13 +188,6 @@ struct Fp0Config {
 // the same bin layout; 8-height variants on problems of at most 128 heights
 // run the 4-height form.
 
-// The banded form's windows are placed with float coordinates, off by less
-// than its 0.05 voxels of margin up to here.
-bool fp0_band_ok(const Geom& g) {
-  constexpr int kMax = 1 << 16;
-  return g.SY <= kMax && g.SX <= kMax && g.PX <= kMax;
-}
-
 // Whether the banded 4-height form splits a run's lines over four warps: when
 // its unsplit blocks fill less than a wave.  A per call, unsplit / split:
 // 32^3 and 128 angles (64 blocks) 16.5 / 8.3 us; 64^3 and 128 (256 blocks)
@@ -250,7 +243,7 @@ Fp0Config fp0_config(const Geom& g, bool vec4, int variant) {
     if (dflt) {
       c.agroup = false;
       if (vec4 && fp0_band_ok(g)) {
-        c.band = g.H <= 16 ? 8 : g.H <= 32 ? 4 : g.H <= 64 ? 2 : 1;
+        c.band = fp0_band_runs(g.H);
         c.split = fp0_band_split(g, c.band);
       }
     }

@@ -163,6 +163,71 @@ __device__ __forceinline__ bool not_finite(const float4 (&acc)[4], int n) {
   return t != t;
 }
 
+__device__ __forceinline__ BandAngle band_angle(const AngleConst& k, const Geom& g,
+                                                const Slab& s) {
+  BandAngle A;
+  A.k = k;
+  A.minor_x = fabsf(k.c) >= fabsf(k.s);
+  A.maj_lo = A.minor_x ? s.y_lo : s.x_lo;
+  A.maj_hi = A.minor_x ? s.y_hi : s.x_hi;
+  A.min_lo = A.minor_x ? 0 : s.yy_lo;
+  A.min_hi = A.minor_x ? g.SX - 1 : s.yy_hi - 1;
+  A.cent_major = A.minor_x ? g.ycent : g.xcent;
+  A.cent_minor = A.minor_x ? g.xcent : g.ycent;
+  A.sh_major = A.minor_x ? k.s : k.c;
+  const float step = A.minor_x ? k.c : k.s;
+  A.inv = 1.0f / step;
+  A.up = step >= 0.0f;
+  return A;
+}
+
+// The sums of G runs from run0 on share `part` of SP of the slab's lines.
+template <int G, int SP>
+__device__ __forceinline__ void band_sums(float4 (&acc)[4], const float* xs, const BandAngle& A,
+                                          const Geom& g, int run0, int part, BandEntry* tab) {
+  int lo = A.maj_lo, hi = A.maj_hi;
+  if (SP > 1) {
+    const int share = (hi - lo + SP - 1) / SP;
+    lo = min(lo + part * share, hi);
+    hi = min(lo + share, hi);
+  }
+  if ((2.0f * A.k.b + 1.0f) * fabsf(A.inv) <= kBandNarrow)
+    band_lines<G, true>(acc, xs, A, g, run0, lo, hi, tab);
+  else
+    band_lines<G, false>(acc, xs, A, g, run0, lo, hi, tab);
+}
+
+// Adds or stores the sums of G runs from run0 on, by the whole warp, after
+// wait(); h: this lane's heights (several runs: of the one chunk).
+template <int G, class Wait, bool VOUT>
+__device__ __forceinline__ void band_write(const float4 (&acc)[4], const float* x, float* y,
+                                           const float* angles, const Geom& g, const Slab& s,
+                                           const BandAngle& A, int run0, int a, int h,
+                                           int accumulate, float4* cand, const Wait& wait) {
+  wait();
+  if (A.maj_lo >= A.maj_hi && accumulate) return;
+  const int lane = threadIdx.x & 31;
+  if (__any_sync(0xffffffffu, not_finite(acc, g.H - h))) {
+    for (int r = 0; r < G; ++r) {
+      __syncwarp();
+      fp_z0_warp<4, 4, 2, Wait, false, VOUT>(x, y, angles, g, 4 * (run0 + r), a,
+                                             G > 1 ? 4 * lane : h, s, accumulate, cand, wait);
+    }
+    return;
+  }
+  const LaneH<4> lh(h, g.H);
+  const int p0 = 4 * (run0 + (G > 1 ? lane / (32 / G) : 0));
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    const int p = A.up ? p0 + b : p0 + 3 - b;
+    if (p < g.PX) {
+      float* row = y + ((size_t)a * g.PX + p) * g.Hy;
+      if constexpr (VOUT) store_lane<4, Wait::coherent>(row, lh, acc[b], accumulate);
+      else store_lane_heights<4, Wait::coherent>(row, lh, acc[b], accumulate, g.H);
+    }
+  }
+}
+
 // Block body.  A warp takes G runs of 4 bins (from run0) of angle a and its
 // lanes' heights from h, on the slab's lines; with SP warps per run set, warp
 // `part` takes every SP-th share of the lines and part 0 writes the sum of all
@@ -174,41 +239,16 @@ __device__ __forceinline__ void fp_band_block(const float* __restrict__ x, float
                                               int run0, int a, int h, const Slab& s, bool has,
                                               int part, int accumulate, BandSmem* sm,
                                               float4 (*sums)[32][4]) {
-  constexpr int LH = 32 / G;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const Wait wait;
-  const LaneH<4> lh(h, g.H);
   float4 acc[4];
 #pragma unroll
   for (int b = 0; b < 4; ++b) acc[b] = vzero<float4>();
   BandAngle A;
-  bool empty = true;
   if (has) {
-    A.k = angle_const(__ldg(angles + a), g.trig);
-    A.minor_x = fabsf(A.k.c) >= fabsf(A.k.s);
-    A.maj_lo = A.minor_x ? s.y_lo : s.x_lo;
-    A.maj_hi = A.minor_x ? s.y_hi : s.x_hi;
-    A.min_lo = A.minor_x ? 0 : s.yy_lo;
-    A.min_hi = A.minor_x ? g.SX - 1 : s.yy_hi - 1;
-    A.cent_major = A.minor_x ? g.ycent : g.xcent;
-    A.cent_minor = A.minor_x ? g.xcent : g.ycent;
-    A.sh_major = A.minor_x ? A.k.s : A.k.c;
-    const float step = A.minor_x ? A.k.c : A.k.s;
-    A.inv = 1.0f / step;
-    A.up = step >= 0.0f;
-    empty = A.maj_lo >= A.maj_hi;
-    int lo = A.maj_lo, hi = A.maj_hi;
-    if (SP > 1) {
-      const int share = (hi - lo + SP - 1) / SP;
-      lo = min(lo + part * share, hi);
-      hi = min(lo + share, hi);
-    }
-    const float* xs = x + lh.s0;
-    if ((2.0f * A.k.b + 1.0f) * fabsf(A.inv) <= kBandNarrow)
-      band_lines<G, true>(acc, xs, A, g, run0, lo, hi, sm->tab);
-    else
-      band_lines<G, false>(acc, xs, A, g, run0, lo, hi, sm->tab);
+    A = band_angle(angle_const(__ldg(angles + a), g.trig), g, s);
+    band_sums<G, SP>(acc, x + (h < g.H ? h : 0), A, g, run0, part, sm->tab);
   }
   if (SP > 1) {
     __syncthreads();
@@ -216,37 +256,38 @@ __device__ __forceinline__ void fp_band_block(const float* __restrict__ x, float
 #pragma unroll
       for (int b = 0; b < 4; ++b) sums[warp][lane][b] = acc[b];
     __syncthreads();
-    if (part > 0) {
-      wait();
-      return;
-    }
+    if (part == 0) {
 #pragma unroll
-    for (int j = 1; j < SP; ++j)
+      for (int j = 1; j < SP; ++j)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) acc[b] = f4_add(acc[b], sums[warp + j][lane][b]);
-    __syncwarp();
-  }
-  wait();
-  if (!has || (empty && accumulate)) return;
-  if (__any_sync(0xffffffffu, not_finite(acc, g.H - h))) {
-    for (int r = 0; r < G; ++r) {
-      // (with several runs per warp all heights are in one chunk from 0)
-      fp_z0_warp<4, 4, 2, NoWait, false, VOUT>(x, y, angles, g, 4 * (run0 + r), a,
-                                               G > 1 ? 4 * lane : h, s, accumulate, sm->cand);
+        for (int b = 0; b < 4; ++b) acc[b] = f4_add(acc[b], sums[warp + j][lane][b]);
       __syncwarp();
     }
+  }
+  if (!has || part > 0) {
+    wait();
     return;
   }
-  const int p0 = 4 * (run0 + (G > 1 ? lane / LH : 0));
-#pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int p = A.up ? p0 + b : p0 + 3 - b;
-    if (p < g.PX) {
-      float* row = y + ((size_t)a * g.PX + p) * g.Hy;
-      if constexpr (VOUT) store_lane<4>(row, lh, acc[b], accumulate);
-      else store_lane_heights<4>(row, lh, acc[b], accumulate, g.H);
-    }
+  band_write<G, Wait, VOUT>(acc, x, y, angles, g, s, A, run0, a, h, accumulate, sm->cand, wait);
+}
+
+// One warp of a batch: as fp_band_block without a split.
+template <int G, class Wait>
+__device__ __forceinline__ void fp_band_warp(const float* __restrict__ x, float* __restrict__ y,
+                                             const float* __restrict__ angles, const Geom& g,
+                                             int run0, int a, int h, const Slab& s,
+                                             BandSmem* sm, const Wait& wait) {
+  if (a >= g.n_ang || 4 * run0 >= g.PX) {  // warp-uniform
+    wait();
+    return;
   }
+  float4 acc[4];
+#pragma unroll
+  for (int b = 0; b < 4; ++b) acc[b] = vzero<float4>();
+  const BandAngle A = band_angle(angle_const(__ldg(angles + a), g.trig), g, s);
+  band_sums<G, 1>(acc, x + (h < g.H ? h : 0), A, g, run0, 0, sm->tab);
+  __syncwarp();
+  band_write<G, Wait, true>(acc, x, y, angles, g, s, A, run0, a, h, 1, sm->cand, wait);
 }
 
 }  // namespace detail

@@ -72,6 +72,15 @@ struct BandLaunch {
 cudaError_t launch_fp_band(const BandLaunch& L, int runs_per_warp, bool split,
                            cudaStream_t stream, int* launches);
 
+// The banded form's windows are placed with float coordinates, off by less
+// than its 0.05 voxels of margin up to here.
+inline bool fp0_band_ok(const Geom& g) {
+  constexpr int kMax = 1 << 16;
+  return g.SY <= kMax && g.SX <= kMax && g.PX <= kMax;
+}
+// Its runs per warp: the fewest lanes that hold the heights (at most 128).
+inline int fp0_band_runs(int H) { return H <= 16 ? 8 : H <= 32 ? 4 : H <= 64 ? 2 : 1; }
+
 // Few heights (vp_thin.cu): the arrays in z_order z.
 cudaError_t launch_forward_thin(const float* x, float* y, const float* angles, const Geom& g,
                                 int z, cudaStream_t stream);
