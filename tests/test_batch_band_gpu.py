@@ -19,7 +19,7 @@ GEOMS = [(20, 26, 31, 29), (50, 40, 13, 150)]  # SY, SX, angles, bins
 
 
 @pytest.mark.parametrize("geoms,heights", [
-    (GEOMS, (8, 16, 20, 32, 36, 64, 100, 128)),
+    (GEOMS, (8, 16, 20, 32, 36, 40, 64, 100, 128)),
     (GEOMS, (132, 140, 192, 196, 400, 448)),
     ([(330, 320, 10, 300)], (160, 416)),  # several slabs
 ])

@@ -217,7 +217,7 @@ __device__ __noinline__ void run_fwd_band_item(const BatchDesc& d, int stage, in
   __syncwarp();
   const int a = d.agroup ? row * BATCH_WARPS + w : row;
   const int set = d.agroup ? u : u * BATCH_WARPS + w;
-  const int h = G > 1 ? (lane % (32 / G)) * 4 : hc * 128 + lane * 4;
+  const int h = G > 1 ? band_height<G>(lane) : hc * 128 + lane * 4;
   fp_band_warp<G>(d.in, d.out, d.angles, d.g, set * G, a, h, slab, &sm.band[w], SlotWait{slot});
   signal_done(slot->counter);
 }
@@ -380,6 +380,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, batch_min_blocks(BODY))
       if (BODY != B_FWD4 || d.band == 0) item_of(run_fwd_item<R, BODY == B_FWD8F>);
       else if (d.band == 1) item_of(run_fwd_band_item<1>);
       else if (d.band == 2) item_of(run_fwd_band_item<2>);
+      else if (d.band == 3) item_of(run_fwd_band_item<3>);
       else if (d.band == 4) item_of(run_fwd_band_item<4>);
       else item_of(run_fwd_band_item<8>);
     } else {

@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(32 * FPB_WARPS, G == 1 ? 6 : 5)
   const int warp = threadIdx.x >> 5;
   const int set = blockIdx.x * (FPB_WARPS / SP) + warp / SP;
   const int a = a_base + blockIdx.y;
-  const int h = G > 1 ? (lane % (32 / G)) * 4 : blockIdx.z * 128 + lane * 4;
+  const int h = G > 1 ? band_height<G>(lane) : blockIdx.z * 128 + lane * 4;
   const bool has = a < g.n_ang && 4 * G * set < g.PX;
   using Wait = std::conditional_t<PDL, PdlWait, NoWait>;
   fp_band_block<G, SP, Wait, VOUT>(x, y, angles, g, set * G, a, h, slab, has,
@@ -79,6 +79,7 @@ cudaError_t launch_fp_band(const BandLaunch& L, int runs_per_warp, bool split,
                            cudaStream_t stream, int* launches) {
   switch (runs_per_warp) {
     case 8: return launch_band_g<8>(L, split, stream, launches);
+    case 3: return launch_band_g<3>(L, split, stream, launches);
     case 4: return launch_band_g<4>(L, split, stream, launches);
     case 2: return launch_band_g<2>(L, split, stream, launches);
     default: return launch_band_g<1>(L, split, stream, launches);

@@ -101,6 +101,18 @@ __device__ __forceinline__ void band_entry(const BandAngle& A, const Geom& g, in
                       !some ? BAND_EMPTY : inside ? BAND_INSIDE : BAND_EDGE, 0);
 }
 
+// With G runs per warp a run has 32 / G lanes of 4 heights; lanes left over
+// (G = 3) follow the last run and hold no heights.
+template <int G>
+__device__ __forceinline__ int band_run(int lane) {
+  return G == 1 ? 0 : min(lane / (32 / G), G - 1);
+}
+template <int G>
+__device__ __forceinline__ int band_height(int lane) {
+  constexpr int LH = 32 / G;
+  return lane < G * LH ? (lane % LH) * 4 : 1 << 29;
+}
+
 // The lines [lo, hi) of the slab for G runs from bin 4 * run0.
 template <int G, bool NARROW>
 __device__ __forceinline__ void band_lines(float4 (&acc)[4], const float* xs, const BandAngle& A,
@@ -109,11 +121,11 @@ __device__ __forceinline__ void band_lines(float4 (&acc)[4], const float* xs, co
   using B = Band<NARROW>;
   constexpr int LB = 32 / G;  // lines per table
   const int lane = threadIdx.x & 31;
-  const BandEntry* mine = tab + (G > 1 ? lane / (32 / G) : 0);
+  const BandEntry* mine = tab + band_run<G>(lane);
   const ptrdiff_t sm = (ptrdiff_t)(A.minor_x ? 1 : g.SX) * g.Hx;  // one voxel along the minor axis
   for (int i0 = lo; i0 < hi; i0 += LB) {
     __syncwarp();
-    if (i0 + lane / G < hi)
+    if (lane < LB * G && i0 + lane / G < hi)
       band_entry<NARROW>(A, g, i0 + lane / G, 4 * (run0 + lane % G), &tab[lane]);
     __syncwarp();
     const int nl = min(LB, hi - i0);
@@ -216,7 +228,7 @@ __device__ __forceinline__ void band_write(const float4 (&acc)[4], const float* 
     return;
   }
   const LaneH<4> lh(h, g.H);
-  const int p0 = 4 * (run0 + (G > 1 ? lane / (32 / G) : 0));
+  const int p0 = 4 * (run0 + band_run<G>(lane));
 #pragma unroll
   for (int b = 0; b < 4; ++b) {
     const int p = A.up ? p0 + b : p0 + 3 - b;

@@ -55,8 +55,8 @@ enum Op : int { OP_FORWARD_Z0 = 0, OP_BACKWARD_Z0 = 1, OP_FORWARD_Z2 = 2, OP_BAC
 int kernel_variant(int op);
 
 // The banded z_order 0 forward (vp_fp_band.cu): one slab launch on angles
-// [a_lo, a_hi); runs_per_warp (1, 2, 4, 8) runs of 4 bins share a warp (more
-// than one: H <= 128 / runs_per_warp), split spreads their lines over the 4
+// [a_lo, a_hi); runs_per_warp (1 to 4, 8) runs of 4 bins share a warp (more
+// than one: H <= 4 * (32 / runs_per_warp)), split spreads their lines over the 4
 // warps of a block.  x's rows are 16-byte aligned.
 struct BandLaunch {
   const float* x;
@@ -78,8 +78,13 @@ inline bool fp0_band_ok(const Geom& g) {
   constexpr int kMax = 1 << 16;
   return g.SY <= kMax && g.SX <= kMax && g.PX <= kMax;
 }
-// Its runs per warp: the fewest lanes that hold the heights (at most 128).
-inline int fp0_band_runs(int H) { return H <= 16 ? 8 : H <= 32 ? 4 : H <= 64 ? 2 : 1; }
+// Its runs per warp: as many as leave a run the lanes for the heights (at most
+// 128).  A (213, 213, 40) and 492 angles 354 us with 2 runs, 293 with 3; 5 runs
+// at 17 to 24 heights gave nothing over 4 (256 x 256 x 20 170 us, 32 heights
+// with 4 163).
+inline int fp0_band_runs(int H) {
+  return H <= 16 ? 8 : H <= 32 ? 4 : H <= 40 ? 3 : H <= 64 ? 2 : 1;
+}
 
 // Few heights (vp_thin.cu): the arrays in z_order z.
 cudaError_t launch_forward_thin(const float* x, float* y, const float* angles, const Geom& g,
