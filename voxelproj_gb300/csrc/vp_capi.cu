@@ -65,9 +65,9 @@ constexpr int kMaxDevices = 64;
 std::mutex g_pool_mutex;
 cudaMemPool_t g_pools[kMaxDevices] = {};
 
-// The second pool, of the padded inputs of z_order 0 calls, keeps at most
-// kPadPoolKeep: more than that goes back to the driver at the next
-// synchronisation.
+// The second pool, of the padded inputs of z_order 0 calls and the workspaces of
+// z_order 2 calls below 32 heights, keeps at most kPadPoolKeep: more than that
+// goes back to the driver at the next synchronisation.
 constexpr uint64_t kPadPoolKeep = (uint64_t)256 << 20;
 cudaMemPool_t g_pad_pools[kMaxDevices] = {};
 
@@ -376,7 +376,8 @@ int run_z2(bool forward, const float* in, float* out, const float* angles, const
       use = false;
     } else {
       cudaMemPool_t pool;
-      cudaError_t e = private_pool(&pool);
+      cudaError_t e = must ? private_pool(&pool)
+                           : device_pool(g_pad_pools, kPadPoolKeep, &pool);
       if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&ws, need, pool, stream);
       if (e != cudaSuccess && must) return finish(e, 0);
       if (e != cudaSuccess) {

@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
 // With SPLIT the four warps of a block take the same voxels and a quarter of
 // the angles each and add up in shared memory (small volumes: enough warps to
 // fill the GPU); else neighbouring rows.  Z2: bins are contiguous, else heights.
-// 512 x 512, 360 angles: one slice 304 -> 137 us, 8 slices 932 -> 652 us.  One
+// 512 x 512, 360 angles: one slice 304 -> 137 us, 8 slices 932 -> 554 us.  One
 // slice issues in 75% of the cycles.
 // ---------------------------------------------------------------------------
 template <int RH, int VR, bool SPLIT, bool Z2, int TRIG>
@@ -297,20 +297,35 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
         const float w0 = tail_area(0.5f - xv, k);
         const float w2 = tail_area(0.5f + xv, k);
         const float w1 = (1.0f - w0) - w2;
-        const bool ok0 = (unsigned)(r - 1) < (unsigned)g.PX;
-        const bool ok1 = (unsigned)r < (unsigned)g.PX;
-        const bool ok2 = (unsigned)(r + 1) < (unsigned)g.PX;
         const float* q = ya + r * yb;
+        if (RH > 1 && __all_sync(0xffffffffu, r >= 1 && r + 1 < g.PX)) {
+          // every lane's three bins on the detector: loads without the zeros and
+          // selects of the guarded ones (8 heights 652 -> 554 us below; one
+          // height 137 -> 148, so not there)
 #pragma unroll
-        for (int h = 0; h < RH; ++h) {
-          if (h < nh) {
-            const float v0 = ok0 ? __ldg(q - yb) : 0.0f;
-            const float v1 = ok1 ? __ldg(q) : 0.0f;
-            const float v2 = ok2 ? __ldg(q + yb) : 0.0f;
-            acc[v][h] = fmaf(w0, v0, acc[v][h]);
-            acc[v][h] = fmaf(w1, v1, acc[v][h]);
-            acc[v][h] = fmaf(w2, v2, acc[v][h]);
-            q += yh;
+          for (int h = 0; h < RH; ++h) {
+            if (h < nh) {
+              acc[v][h] = fmaf(w0, __ldg(q - yb), acc[v][h]);
+              acc[v][h] = fmaf(w1, __ldg(q), acc[v][h]);
+              acc[v][h] = fmaf(w2, __ldg(q + yb), acc[v][h]);
+              q += yh;
+            }
+          }
+        } else {
+          const bool ok0 = (unsigned)(r - 1) < (unsigned)g.PX;
+          const bool ok1 = (unsigned)r < (unsigned)g.PX;
+          const bool ok2 = (unsigned)(r + 1) < (unsigned)g.PX;
+#pragma unroll
+          for (int h = 0; h < RH; ++h) {
+            if (h < nh) {
+              const float v0 = ok0 ? __ldg(q - yb) : 0.0f;
+              const float v1 = ok1 ? __ldg(q) : 0.0f;
+              const float v2 = ok2 ? __ldg(q + yb) : 0.0f;
+              acc[v][h] = fmaf(w0, v0, acc[v][h]);
+              acc[v][h] = fmaf(w1, v1, acc[v][h]);
+              acc[v][h] = fmaf(w2, v2, acc[v][h]);
+              q += yh;
+            }
           }
         }
       }
