@@ -163,19 +163,21 @@ __global__ void __launch_bounds__(32 * BPB_WARPS)
 // PDL: the launch follows another run launch of the same call
 // programmatically (launch_ex), so its warps wait for that launch before they
 // add into x; a call's first launch keeps the form without the wait.
-// VOUT: see bp_runs_warp.
+// VOUT: see bp_runs_warp.  band_rows: order of the blocks (tile_order).
 template <int PASS, int R, bool ADD = false, bool FULL = false, bool PDL = false,
           bool VOUT = true>
 __global__ void __launch_bounds__(32 * BPR_WARPS, R == 8 ? 5 : 0)
     bp_z0_runs_kernel(const float* __restrict__ y, float* __restrict__ x,
                       const float* __restrict__ angles, Geom g, int nrun_major, int run_base,
-                      int run_end, int row_end, int accumulate,
+                      int run_end, int row_end, int accumulate, unsigned band_rows,
                       const float* __restrict__ addend = nullptr) {
   __shared__ RunEntry tab[BPR_WARPS][BPR_CHUNK];
   __shared__ int alist[BPR_WARPS][BPR_LIST];
   const int lane = threadIdx.x;
   const int w = threadIdx.y;
-  const int run = run_base + blockIdx.x * BPR_WARPS + w;
+  const unsigned nx = PASS == 0 ? nrun_major : (unsigned)nrun_major / BPR_WARPS;
+  const unsigned tile = tile_order(blockIdx.x, nx, gridDim.x, band_rows);
+  const int run = run_base + tile * BPR_WARPS + w;
   // A programmatic launch of the next class may start as this one's last
   // blocks run; each warp waits for the launch before it only to add its
   // sums into x.  Warp 0 of every block has a run inside the range (the grid
@@ -188,7 +190,7 @@ __global__ void __launch_bounds__(32 * BPR_WARPS, R == 8 ? 5 : 0)
   if (run >= run_end) return;  // warp-uniform; all shared state is per warp
   int xi0, yi0;
   run_origin<PASS>(run, nrun_major, &xi0, &yi0);
-  if (yi0 >= row_end) return;
+  if (yi0 >= row_end || (PASS == 1 && xi0 >= g.SX)) return;
   using Wait = std::conditional_t<PDL, PdlWait, NoWait>;
   bp_runs_warp<PASS, R, Wait, ADD, FULL, VOUT>(y, x, angles, g, xi0, yi0,
                                          blockIdx.y * 32 * R + lane * 4, accumulate, tab[w],
@@ -474,22 +476,24 @@ cudaError_t launch_bp_z0_runs_h(const float* y, float* x, const float* angles, c
   const long long b0 = (long long)row_lo * nmaj0;
   const long long e0 = (long long)ceil_div(row_hi, RUN) * RUN * nmaj0;
   const float* no_addend = nullptr;
+  const unsigned bands0 = bp_band_rows(g, 0, R), bands1 = bp_band_rows(g, 1, R);
+  const int ncol1 = class1_columns(g, bands1);
   if (e0 > b0) {
     const dim3 grid(ceil_div(e0 - b0, BPR_WARPS), hchunks);
     cudaError_t e =
         programmatic
             ? launch_ex(bp_z0_runs_kernel<0, R, false, FULL, true, VOUT>, grid, block, 0, stream,
                         true, y, x, angles, g, nmaj0, (int)b0, (int)e0, row_hi, g.accumulate,
-                        no_addend)
+                        bands0, no_addend)
             : launch_ex(bp_z0_runs_kernel<0, R, false, FULL, false, VOUT>, grid, block, 0, stream,
                         false, y, x, angles, g, nmaj0, (int)b0, (int)e0, row_hi, g.accumulate,
-                        no_addend);
+                        bands0, no_addend);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     programmatic = true;
   }
-  const long long b1 = (long long)(row_lo / RUN) * g.SX;
-  const long long e1 = (long long)ceil_div(row_hi, RUN) * g.SX;
+  const long long b1 = (long long)(row_lo / RUN) * ncol1;
+  const long long e1 = (long long)ceil_div(row_hi, RUN) * ncol1;
   if (e1 > b1) {
     const dim3 grid(ceil_div(e1 - b1, BPR_WARPS), hchunks);
     // the class-1 launch follows the class-0 one whenever there is one (an
@@ -503,18 +507,18 @@ cudaError_t launch_bp_z0_runs_h(const float* y, float* x, const float* angles, c
     // (containers come in whole float4: backward_z0_rows_can_add)
     if (VOUT && addend)
       e = programmatic ? launch_ex(bp_z0_runs_kernel<1, R, true, FULL, true>, grid, block, 0,
-                                   stream, true, y, x, angles, g, g.SX, (int)b1, (int)e1,
-                                   row_hi, 1, addend)
+                                   stream, true, y, x, angles, g, ncol1, (int)b1, (int)e1,
+                                   row_hi, 1, bands1, addend)
                        : launch_ex(bp_z0_runs_kernel<1, R, true, FULL, false>, grid, block, 0,
-                                   stream, false, y, x, angles, g, g.SX, (int)b1, (int)e1,
-                                   row_hi, 1, addend);
+                                   stream, false, y, x, angles, g, ncol1, (int)b1, (int)e1,
+                                   row_hi, 1, bands1, addend);
     else
       e = programmatic ? launch_ex(bp_z0_runs_kernel<1, R, false, FULL, true, VOUT>, grid, block, 0,
-                                   stream, true, y, x, angles, g, g.SX, (int)b1, (int)e1,
-                                   row_hi, 1, no_addend)
+                                   stream, true, y, x, angles, g, ncol1, (int)b1, (int)e1,
+                                   row_hi, 1, bands1, no_addend)
                        : launch_ex(bp_z0_runs_kernel<1, R, false, FULL, false, VOUT>, grid, block,
-                                   0, stream, false, y, x, angles, g, g.SX, (int)b1, (int)e1,
-                                   row_hi, 1, no_addend);
+                                   0, stream, false, y, x, angles, g, ncol1, (int)b1, (int)e1,
+                                   row_hi, 1, bands1, no_addend);
     if (e == cudaSuccess) e = cudaGetLastError();
     return e;
   }

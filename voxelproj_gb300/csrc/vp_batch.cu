@@ -95,8 +95,10 @@ struct BatchDesc {
   // (vp_fp_band.cuh), 0 = candidate lists; an item column is then one set of
   // runs (agroup) or one per warp
   int band;
-  // run adjoint: runs and run groups of each class
-  int nruns0, groups0, nruns1, groups1;
+  // run adjoint: runs and run groups of each class, class-1 columns (runs per
+  // band), and the order the groups are taken in (tile_order)
+  int nruns0, groups0, nruns1, groups1, ncol1;
+  unsigned bands0, bands1;
   // block adjoint: blocks along x, blocks, block groups
   int nbx, nblocks, bgroups;
 };
@@ -232,14 +234,16 @@ __device__ __noinline__ void run_fwd_band_item(const BatchDesc& d, int stage, in
 // took a chunk's first class-1 items spun while its last class-0 items ran.
 // FULL: the part's heights are whole 256-height chunks (R = 8).
 template <int R, bool FULL>
-__device__ __forceinline__ void run_bwd_runs_item(const BatchDesc& d, int stage, int grp,
+__device__ __forceinline__ void run_bwd_runs_item(const BatchDesc& d, int stage, int item,
                                                   int hc, RunsSmem& sm, int w, int lane,
                                                   unsigned* counters, int* error,
                                                   const WaitLimits& lim) {
   unsigned* tiles = counters + d.counter_base + (size_t)hc * d.groups0;
-  const int run = grp * BATCH_WARPS + w;
   const int h = hc * 32 * R + lane * 4;
   const int nmaj = (d.g.SX + RUN - 1) / RUN;
+  const int grp = stage == 0 ? (int)tile_order(item, nmaj, d.groups0, d.bands0)
+                             : (int)tile_order(item, d.ncol1 / BPR_WARPS, d.groups1, d.bands1);
+  const int run = grp * BATCH_WARPS + w;
   if (stage == 0) {
     int xi0, yi0;
     run_origin<0>(run, nmaj, &xi0, &yi0);
@@ -248,8 +252,9 @@ __device__ __forceinline__ void run_bwd_runs_item(const BatchDesc& d, int stage,
                                               sm.tab[w], sm.alist[w]);
     signal_done(tiles + grp);
   } else if (run < d.nruns1) {
-    const int x = run % d.g.SX;
-    const int band = run / d.g.SX;
+    const int x = run % d.ncol1;
+    const int band = run / d.ncol1;
+    if (x >= d.g.SX) return;  // (warp-uniform; class-1 items signal nothing)
     const StageWait wt{tiles + band * nmaj + x / RUN, (unsigned)BATCH_WARPS + lim.extra, error,
                        lim.spins};
     bp_runs_warp<1, R, StageWait, false, FULL>(d.in, d.out, d.angles, d.g, x, band * RUN, h, 1,
@@ -510,7 +515,10 @@ int part_desc(const vp_batch_problem& p, const vp::Geom& g, const float* in, flo
     // class-0 runs in bands of RUN rows (run_origin), rows padded to the band
     d->nruns0 = (int)vp::ceil_div_u(g.SX, vp::detail::RUN) *
                 (int)vp::ceil_div_u(g.SY, vp::detail::RUN) * vp::detail::RUN;
-    d->nruns1 = g.SX * (int)vp::ceil_div_u(g.SY, vp::detail::RUN);
+    d->bands0 = vp::detail::bp_band_rows(g, 0, R);
+    d->bands1 = vp::detail::bp_band_rows(g, 1, R);
+    d->ncol1 = vp::detail::class1_columns(g, d->bands1);
+    d->nruns1 = d->ncol1 * (int)vp::ceil_div_u(g.SY, vp::detail::RUN);
     d->groups0 = (int)vp::ceil_div_u(d->nruns0, vp::BATCH_WARPS);
     d->groups1 = (int)vp::ceil_div_u(d->nruns1, vp::BATCH_WARPS);
     d->per_chunk = (long long)d->groups0 + d->groups1;

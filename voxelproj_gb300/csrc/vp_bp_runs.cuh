@@ -74,6 +74,45 @@ __device__ __forceinline__ void run_origin(int run, int nrun_major, int* xi0, in
   }
 }
 
+// Tiles (blocks of BPR_WARPS runs) of a class in the order they are taken:
+// row by row, or with rows > 0 by bands of `rows` tile rows, column by column
+// within a band.  b: place in that order; nx, n: tiles per row, tiles.
+__host__ __device__ __forceinline__ unsigned tile_order(unsigned b, unsigned nx, unsigned n,
+                                                        unsigned rows) {
+  if (rows == 0) return b;
+  const unsigned band = b / (rows * nx) * rows;  // the band's first tile row
+  const unsigned ny = n / nx - band;
+  const unsigned left = ny < rows ? ny : rows;
+  const unsigned q = b - band * nx;
+  return (band + q % left) * nx + q / left;
+}
+
+// Tile rows per band for tile_order; class cls, R heights per lane; 0 = row by
+// row.
+// What matters is the part of the sinogram that the resident blocks (760 at
+// R = 8) sweep together: they drift apart in angle, so it is every class angle
+// times the bins their voxels project to.  While the class's half of a height
+// chunk's sinogram fits in one die's half of L2 (64 MB) any order does, and row
+// by row gives class 0 slightly better L1 reuse.  Past it, whole tile rows
+// reread it from DRAM: a 6 tile row strip projects to all 512 bins at most
+// class-1 angles, a 20 x 38 or 64 x 12 patch to a fraction of them (class-1
+// windows lie along x, so its patches are tall; class-0 ones wide).  A^T at
+// 512^3 and 1024 angles, 256 MB per class: 26.6 ms (up to 28.8 by run) -> 22.5;
+// 384 angles 9.2 -> 8.5 ms; 1024 x 1024 x 256 and 360 angles 18.8 -> 15.9;
+// 256^3 and 720 angles (94 MB) 2.17 -> 2.10; 512 x 512 x 128 and 1440 angles
+// 10.6 -> 9.4.  At 192 angles (50 MB) 4.33 row by row, 4.38 ms in bands.  Bands
+// of 28 and 28 took 22.8 ms, 18 and 43 22.7, 20 and 128 23.9, 8 and 64 23.0.
+// Bands need blocks that are tiles: class-1 columns are then numbered in whole
+// blocks (class1_columns), and warps past SX have no run.
+constexpr size_t kBpRowOrderBytes = (size_t)144 << 20;
+inline unsigned bp_band_rows(const Geom& g, int cls, int R) {
+  const size_t sino = (size_t)g.n_ang * g.PX * (g.H < 32 * R ? g.H : 32 * R) * sizeof(float);
+  return sino <= kBpRowOrderBytes ? 0 : cls == 0 ? 20 : 64;
+}
+inline int class1_columns(const Geom& g, unsigned band_rows) {
+  return band_rows ? (g.SX + BPR_WARPS - 1) / BPR_WARPS * BPR_WARPS : g.SX;
+}
+
 template <int PASS>
 __device__ __forceinline__ bool in_class(float phi, int trig) {
   float s, c;
