@@ -164,23 +164,14 @@ int host_entry(bool z2, const float* x, int64_t x0, int64_t x1, int64_t x2, cons
 namespace {
 
 // z_order 0 input whose rows are not whole, aligned float4: a copy with rows
-// padded to a multiple of 4 heights lets the float4 kernels run (their
-// epilogues write such outputs by single heights).  The copy costs one read
-// and one write of the input; the scalar kernels it replaces held one height
-// per lane: (301, 257, 203) and 181 angles, A 3.76 -> 1.16 ms, A^T 3.00 ->
-// 0.81 ms.  The adjoint from 33 heights on: up to 32, one scalar chunk per warp
-// does the float4 form's work.  Not under stream capture, and not without memory for
-// the copy: the scalar kernels run then, as they do for other variants.
-constexpr int kPadMinHeights = 33;
-
+// padded to a multiple of 4 heights where that pays (z0_pads).  Not under stream
+// capture, and not without memory for the copy: the scalar kernels run then.
 // The padded copy of `in` (rows x Hin floats) in *copy, or nullptr when the
 // call is to run on `in` itself.
 cudaError_t padded_input(int op, const float* in, int64_t rows, int Hin, const vp::Geom& g,
                          cudaStream_t stream, float** copy, int* Hp) {
   *copy = nullptr;
-  if (vp::kernel_variant(op) != 0 ||
-      (op == vp::OP_FORWARD_Z0 ? vp::z0_forward_thin(g) : g.H < kPadMinHeights) ||
-      (Hin % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0))
+  if (!vp::z0_pads(op, g) || (Hin % 4 == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0))
     return cudaSuccess;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   cudaError_t e = cudaStreamIsCapturing(stream, &cap);

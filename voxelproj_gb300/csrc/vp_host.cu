@@ -55,8 +55,14 @@ namespace vp {
 namespace {
 
 constexpr int kMaxDevices = 64;
-constexpr int kAdjointSlabs = 12;     // adjoint row slabs per call
-constexpr int kZ2AdjointSlabs = 8;    // row slabs of the z_order 2 adjoint's last chunk
+constexpr int kAdjointSlabs = 12;     // adjoint row slabs per call at most
+constexpr int kZ2AdjointSlabs = 8;    // row slabs of the z_order 2 adjoint's last chunk at most
+// Blocks of one class launch that a row slab of an adjoint should hold at least
+// (5 resident blocks per SM: 1.5 waves).  Smaller slabs leave the GPU idle for
+// longer than they save in copies.  Host calls with and without the limit:
+// 256^3 and 360 angles 1.64 / 1.88 ms, (256, 256, 128) 0.93 / 1.31, 128 x 128 x
+// 100 and 200 0.30 / 0.65; 384 x 384 x 300 the same (4.01).
+constexpr long long kSlabBlocks = 1140;
 constexpr int kForwardAngleGroups = 4;  // groups of the forward's last slab
 // Forward angles sent home early: |phi| at most this many radians, and
 // |cos phi| - |sin phi| at least this margin, far above the error of the
@@ -213,12 +219,20 @@ struct FwdZ0IO {  // z_order 0 host arrays: contiguous row and angle blocks
   float* xd;
   float* yd;
   float* yc;
+  float* raw;     // null, or where the rows arrive to be padded into xd (Hp heights)
+  int Hp;
+  int* launches;  // counts the padding kernels
   size_t row_elems() const { return (size_t)g.SX * g.Hx; }
   size_t ang_elems() const { return (size_t)g.PX * g.Hy; }
   cudaError_t rows_in(int lo, int hi, cudaStream_t copy) const {
     const size_t off = (size_t)lo * row_elems();
-    return cudaMemcpyAsync(xd + off, x_host + off, (size_t)(hi - lo) * row_elems() * sizeof(float),
-                           cudaMemcpyDefault, copy);
+    float* dst = (raw ? raw : xd) + off;
+    VP_TRY(cudaMemcpyAsync(dst, x_host + off, (size_t)(hi - lo) * row_elems() * sizeof(float),
+                           cudaMemcpyDefault, copy));
+    if (!raw) return cudaSuccess;
+    *launches += 1;
+    return pad_heights(dst, xd + (size_t)lo * g.SX * Hp, (long long)(hi - lo) * g.SX, g.Hx, Hp,
+                       g.H, copy);
   }
   cudaError_t container_in(cudaStream_t copy) const {
     if (!g.accumulate) return cudaSuccess;
@@ -438,12 +452,20 @@ struct BwdZ0IO {  // z_order 0 host arrays: contiguous row and angle blocks
   float* yd;
   float* xd;
   float* xc;
+  float* raw;     // null, or where the angles arrive to be padded into yd (Hp heights)
+  int Hp;
+  int* launches;  // counts the padding kernels
   size_t row_elems() const { return (size_t)g.SX * g.Hx; }
   size_t ang_elems() const { return (size_t)g.PX * g.Hy; }
   cudaError_t angles_in(int a0, int a1, cudaStream_t copy) const {
     const size_t off = (size_t)a0 * ang_elems();
-    return cudaMemcpyAsync(yd + off, y_host + off, (size_t)(a1 - a0) * ang_elems() * sizeof(float),
-                           cudaMemcpyDefault, copy);
+    float* dst = (raw ? raw : yd) + off;
+    VP_TRY(cudaMemcpyAsync(dst, y_host + off, (size_t)(a1 - a0) * ang_elems() * sizeof(float),
+                           cudaMemcpyDefault, copy));
+    if (!raw) return cudaSuccess;
+    *launches += 1;
+    return pad_heights(dst, yd + (size_t)a0 * g.PX * Hp, (long long)(a1 - a0) * g.PX, g.Hy, Hp,
+                       g.H, copy);
   }
   cudaError_t container_rows_in(int lo, int hi, cudaStream_t copy) const {
     if (!g.accumulate) return cudaSuccess;
@@ -462,6 +484,16 @@ struct BwdZ0IO {  // z_order 0 host arrays: contiguous row and angle blocks
   }
 };
 
+// Rows per adjoint slab: about SY / slabs, at least kSlabBlocks blocks of 4 x 4
+// voxels by up to 256 heights, a multiple of step.
+int adjoint_slab_rows(const Geom& g, int slabs, int step) {
+  const long long per_step = (long long)step * ((g.SX + 3) / 4) * ((g.H + 255) / 256);
+  const long long least = (4 * kSlabBlocks + per_step - 1) / per_step;
+  long long steps = ((g.SY + slabs - 1) / slabs + step - 1) / step;
+  if (steps < least) steps = least;
+  return steps * step < g.SY ? (int)(steps * step) : g.SY;
+}
+
 // The adjoint's pipeline on device y (yd) and x (xd) in z_order 0 layout of
 // geometry g; io moves the host arrays.  Called under g_mutex.
 template <class IO>
@@ -470,13 +502,8 @@ cudaError_t backward_pipeline(const IO& io, const float* angles, const Geom& g, 
                               int* launches) {
   const size_t ang_elems = (size_t)g.PX * g.Hy;
   const size_t x_elems = (size_t)g.SY * g.SX * g.Hx;
-  // rows per slab: a multiple of the adjoint's row step, about SY / kAdjointSlabs
   const int step = backward_z0_row_step(yd, xd, g);
-  int rows = g.SY;
-  if (step > 0) {
-    rows = (g.SY + kAdjointSlabs - 1) / kAdjointSlabs;
-    rows = (rows + step - 1) / step * step;
-  }
+  const int rows = step > 0 ? adjoint_slab_rows(g, kAdjointSlabs, step) : g.SY;
   const int nslabs = (g.SY + rows - 1) / rows;
   // the first sixth of the angles runs over the whole volume first, while
   // the rest of the sinogram arrives (at 512^3 with 192 angles, 12 slabs
@@ -556,48 +583,115 @@ cudaError_t backward_pipeline(const IO& io, const float* angles, const Geom& g, 
   return cudaStreamWaitEvent(s, ev_out, 0);  // s ends after the last row is home
 }
 
+// A z_order 0 call of few heights (vp_thin.cu), one step after another: its
+// arrays are small next to its kernel, and the pipelines' pieces would run the
+// scalar kernels.  A (512, 512, 1) and 360 angles 3273 -> 420 us (device
+// buffers 350), (384, 384, 3) and 300 1784 -> 400.
+cudaError_t z0_thin_host(bool forward, const float* in_host, float* out_host,
+                         const float* angles, const Geom& g, cudaMemPool_t pool, cudaStream_t s,
+                         int* launches) {
+  const size_t x_elems = (size_t)g.SY * g.SX * g.Hx;
+  const size_t y_elems = (size_t)g.n_ang * g.PX * g.Hy;
+  const size_t n_in = forward ? x_elems : y_elems, n_out = forward ? y_elems : x_elems;
+  Buffers buf(s);
+  return guarded([&]() -> cudaError_t {
+    float *in = nullptr, *out = nullptr, *as = nullptr;
+    const float* ad = nullptr;
+    VP_TRY(buf.get(pool, n_in * sizeof(float), &in));
+    VP_TRY(buf.get(pool, n_out * sizeof(float), &out));
+    VP_TRY(alloc_angles(angles, g, buf, pool, &ad, &as));
+    VP_TRY(copy_angles(as, angles, g, s));
+    VP_TRY(cudaMemcpyAsync(in, in_host, n_in * sizeof(float), cudaMemcpyDefault, s));
+    Geom gk = g;
+    if (g.accumulate) {
+      VP_TRY(cudaMemcpyAsync(out, out_host, n_out * sizeof(float), cudaMemcpyDefault, s));
+    } else if (g.H < (forward ? g.Hy : g.Hx)) {
+      // heights past the input's extent are not written: start from zero
+      VP_TRY(cudaMemsetAsync(out, 0, n_out * sizeof(float), s));
+      gk.accumulate = 1;
+    }
+    if (forward) {
+      VP_TRY(launch_forward_thin(in, out, ad, gk, 0, s));
+      *launches += launches_forward_thin(gk);
+    } else {
+      VP_TRY(launch_backward_thin(in, out, ad, gk, 0, s));
+      *launches += 1;
+    }
+    return cudaMemcpyAsync(out_host, out, n_out * sizeof(float), cudaMemcpyDefault, s);
+  }, s);
+}
+
+// The device buffer of a pipeline's input: rows x Hin floats, or, where the
+// float4 kernels want padded rows (z0_pads) and there is memory for both, rows x
+// Hp with *raw to arrive in.
+cudaError_t input_buffer(int op, const Geom& g, size_t rows, int Hin, Buffers& buf,
+                         cudaMemPool_t pool, float** dev, float** raw, int* Hp) {
+  *raw = nullptr;
+  *Hp = Hin;
+  VP_TRY(buf.get(pool, rows * Hin * sizeof(float), dev));
+  if (Hin % 4 == 0 || !z0_pads(op, g)) return cudaSuccess;
+  float* padded = nullptr;
+  const int hp = (g.H + 3) / 4 * 4;
+  if (buf.get(pool, rows * hp * sizeof(float), &padded) != cudaSuccess) {
+    cudaGetLastError();  // no room: run on the input itself
+    return cudaSuccess;
+  }
+  *raw = *dev;
+  *dev = padded;
+  *Hp = hp;
+  return cudaSuccess;
+}
+
 }  // namespace
 
 cudaError_t forward_z0_host(const float* x_host, float* y_host, const float* angles,
                             const Geom& g, cudaMemPool_t pool, cudaStream_t s, int* launches) {
   std::lock_guard<std::mutex> lock(g_mutex);
-  const size_t x_elems = (size_t)g.SY * g.SX * g.Hx;
+  if (kernel_variant(OP_FORWARD_Z0) == 0 && z0_forward_thin(g))
+    return z0_thin_host(true, x_host, y_host, angles, g, pool, s, launches);
   const size_t y_elems = (size_t)g.n_ang * g.PX * g.Hy;
   Buffers buf(s);
   return guarded([&]() -> cudaError_t {
-    float *xd = nullptr, *yd = nullptr, *yc = nullptr, *as = nullptr;
+    float *xd = nullptr, *yd = nullptr, *yc = nullptr, *as = nullptr, *raw = nullptr;
     const float* ad = nullptr;
-    VP_TRY(buf.get(pool, x_elems * sizeof(float), &xd));
+    Geom gd = g;  // with the device input's heights per row
     VP_TRY(buf.get(pool, y_elems * sizeof(float), &yd));
     if (g.accumulate) VP_TRY(buf.get(pool, y_elems * sizeof(float), &yc));
     VP_TRY(alloc_angles(angles, g, buf, pool, &ad, &as));
-    const FwdZ0IO io{x_host, y_host, g, xd, yd, yc};
-    return forward_pipeline(io, angles, g, xd, yd, as, ad, s, launches);
+    VP_TRY(input_buffer(OP_FORWARD_Z0, g, (size_t)g.SY * g.SX, g.Hx, buf, pool, &xd, &raw,
+                        &gd.Hx));
+    const FwdZ0IO io{x_host, y_host, g, xd, yd, yc, raw, gd.Hx, launches};
+    return forward_pipeline(io, angles, gd, xd, yd, as, ad, s, launches);
   }, s);
 }
 
 cudaError_t backward_z0_host(const float* y_host, float* x_host, const float* angles,
                              const Geom& g, cudaMemPool_t pool, cudaStream_t s, int* launches) {
   std::lock_guard<std::mutex> lock(g_mutex);
+  if (kernel_variant(OP_BACKWARD_Z0) == 0 && z0_backward_thin(g))
+    return z0_thin_host(false, y_host, x_host, angles, g, pool, s, launches);
   const size_t x_elems = (size_t)g.SY * g.SX * g.Hx;
-  const size_t y_elems = (size_t)g.n_ang * g.PX * g.Hy;
   Buffers buf(s);
   return guarded([&]() -> cudaError_t {
-    float *xd = nullptr, *yd = nullptr, *xc = nullptr, *as = nullptr;
+    float *yd = nullptr, *xd = nullptr, *xc = nullptr, *as = nullptr, *raw = nullptr;
     const float* ad = nullptr;
-    VP_TRY(buf.get(pool, y_elems * sizeof(float), &yd));
+    Geom gd = g;  // with the device input's heights per row
     VP_TRY(buf.get(pool, x_elems * sizeof(float), &xd));
     if (g.accumulate) VP_TRY(buf.get(pool, x_elems * sizeof(float), &xc));
     VP_TRY(alloc_angles(angles, g, buf, pool, &ad, &as));
-    const BwdZ0IO io{y_host, x_host, g, yd, xd, xc};
-    return backward_pipeline(io, angles, g, yd, xd, as, ad, s, launches);
+    VP_TRY(input_buffer(OP_BACKWARD_Z0, g, (size_t)g.n_ang * g.PX, g.Hy, buf, pool, &yd, &raw,
+                        &gd.Hy));
+    const BwdZ0IO io{y_host, x_host, g, yd, xd, xc, raw, gd.Hy, launches};
+    return backward_pipeline(io, angles, gd, yd, xd, as, ad, s, launches);
   }, s);
 }
 
 // The z_order 2 adjoint with host arrays, by chunks of heights, whose
 // sinogram and volume blocks are contiguous: chunks of 256 heights (the
-// 8-heights-per-lane kernels' chunk) from 512 heights up, else halves.  With
-// the transposed path (32 heights and more):
+// 8-heights-per-lane kernels' chunk) above 256 heights, halves from 129, one
+// chunk up to 128, which the 4-height kernels project at once: (256, 256, 101)
+// and 360 angles 1.10 against 1.76 ms in halves, (384, 384, 300) and 300 4.07
+// against 5.07.  With the transposed path (32 heights and more):
 //   copy stream:  the chunks' sinograms in order, each container after the
 //                 next chunk's sinogram (a projection needs only its input)
 //   kernel streams (alternating by chunk, one projection at a time): the
@@ -615,8 +709,8 @@ cudaError_t z2_backward_chunked(const float* y_host, float* x_host, const float*
   const size_t vox = (size_t)g.SY * g.SX, bins = (size_t)g.n_ang * g.PX;
   const int H = g.H;
   int Hc = H;
-  if (H >= 512) Hc = 256;
-  else if (H > 64) Hc = ((H + 1) / 2 + 3) / 4 * 4;
+  if (H > 256) Hc = 256;
+  else if (H > 128) Hc = ((H + 1) / 2 + 3) / 4 * 4;
   const int nchunks = (H + Hc - 1) / Hc;
   Geom gc = g;  // a full chunk
   gc.H = gc.Hx = gc.Hy = Hc;
@@ -647,11 +741,7 @@ cudaError_t z2_backward_chunked(const float* y_host, float* x_host, const float*
       gl.H = gl.Hx = gl.Hy = (int)(((size_t)gl.H + 3) / 4 * 4);
       const float* xtl = ws[(nchunks - 1) & 1];
       const int step = backward_z0_row_step(xtl + vox * gl.H, xtl, gl);
-      int rows = g.SY;
-      if (step > 0) {
-        rows = (g.SY + kZ2AdjointSlabs - 1) / kZ2AdjointSlabs;
-        rows = (rows + step - 1) / step * step;
-      }
+      const int rows = step > 0 ? adjoint_slab_rows(gl, kZ2AdjointSlabs, step) : g.SY;
       for (int q = 0; q < g.SY;) {
         q = q + rows < g.SY ? q + rows : g.SY;
         scut.push_back(q);

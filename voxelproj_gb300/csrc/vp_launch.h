@@ -105,6 +105,15 @@ inline bool z0_backward_thin(const Geom& g) { return g.H <= 7 && g.H % 4 != 0; }
 // 16-byte aligned, Hd a multiple of 4 (vp_z2.cu).
 cudaError_t pad_heights(const float* src, float* dst, long long rows, int Hs, int Hd, int H,
                         cudaStream_t stream);
+// Whether a call whose input rows are not whole float4 takes a padded copy, so
+// that the float4 kernels run (their epilogues write such outputs by single
+// heights).  The copy costs one read and one write of the input; the scalar
+// kernels it replaces held one height per lane: (301, 257, 203) and 181 angles,
+// A 3.76 -> 1.16 ms, A^T 3.00 -> 0.81 ms.  The adjoint from 33 heights on: up
+// to 32, one scalar chunk per warp does the float4 form's work.
+inline bool z0_pads(int op, const Geom& g) {
+  return kernel_variant(op) == 0 && (op == OP_FORWARD_Z0 ? !z0_forward_thin(g) : g.H > 32);
+}
 
 // z_order 2 through the z_order 0 kernels (vp_z2.cu).
 // From 32 heights on always; from 5 on the forward does where it has the
