@@ -5,13 +5,15 @@
 // uploads a descriptor table (the only allocations: the table, the stage
 // counters and an error flag).  vp_batch_run resets the counters and, for
 // each body present (forward or run adjoint, 4 or 8 heights per lane, the
-// 8-height forms also on whole 256-height chunks), launches one persistent kernel with a full wave of blocks (SMs x resident
-// blocks).
+// 8-height forms also on whole 256-height chunks), launches one persistent
+// kernel with a full wave of blocks (SMs x resident blocks).
 // Each block repeatedly takes the next item from a global counter, finds its
 // problem by binary search and runs the same per-warp bodies, with the same
 // heights per lane and the same volume slabs, as the single-problem kernel
 // of the problem's variant:
-//   forward item = (problem, height chunk, volume slab, angle, 4 bin runs)
+//   forward item = (problem, height chunk, volume slab, angle, 4 bin runs; or
+//                  4 angles, one bin run), banded 4-height parts (vp_fp_band.cuh)
+//                  with several runs per warp
 //   adjoint item = (problem, height chunk, angle class, 4 voxel runs)
 //                  or, variant 4, (problem, chunk, 4 voxel blocks of 2x2)
 // A height chunk is 32 lanes x 4 or 8 heights.  Items are numbered problem
@@ -26,8 +28,8 @@
 // itself done after writing, and a task of stage s > 0 waits, just before its
 // read-modify-write, until what it adds to is complete, then reads the output
 // past L1: for the forward, the same output tile (height chunk, angle, bin
-// group) at stage s-1, on the tile's counter; for the adjoint, all of stage
-// s-1, on the stage's counter.  Items are taken in increasing order, so every
+// group) at stage s-1, on the tile's counter; for the adjoint, the class-0
+// item of its 4 x 4 voxel tile, on that item's counter.  Items are taken in increasing order, so every
 // task a waiter depends on was taken earlier by a block that is already
 // running: the wait always ends.  It is bounded anyway: after ~4 s of spinning
 // it records an error (vp_batch_error) and writes regardless.  The bound is a

@@ -177,16 +177,17 @@ struct Fp0Config {
 // per block, the volume staged through shared memory by tensor copies
 // (vp_fp_staged.cuh); 19 = the aligned angle groups with plain loads; 21 /
 // 22 / 23 = as 16 with 128 / 32 / 256 MB slabs.  The default (0) is 16 with
-// 8 heights per lane and 10's layout (neighbouring bins) in the 4-height
-// form.  Measured A per call with programmatic launches between the slab
+// 8 heights per lane; at most 128 heights, and a rest of 129 to 192 in two
+// parts, run the banded 4-height form (vp_fp_band.cuh), at most 4 heights the
+// kernel of vp_thin.cu.  Measured A per call with programmatic launches between the slab
 // launches, variants 16 / 21 / 22 / 23: 512^3 and 192 angles 6.66 / 6.73 /
 // 7.05 / 7.12 ms; 1024 angles 32.98 / 33.89 / 35.06 ms; 256^3 and 360 angles
 // 1.534 / 1.585 / 1.551 ms; 384^3 and 641 angles 10.54 / 10.50 / 11.01 ms.
 // (Without them 21 led: 6.94 against 7.02 ms at 512^3, the extra slab
 // launches' tails costing more than the volume's better L2 residency.)
-// Heights not in float4 run the scalar form of
-// the same bin layout; 8-height variants on problems of at most 128 heights
-// run the 4-height form.
+// Volume rows not in float4 run the scalar form of
+// the same bin layout (the default gets them padded: z0_pads); 8-height
+// variants on problems of at most 128 heights run the 4-height form.
 
 // Whether the banded 4-height form splits a run's lines over four warps: when
 // its unsplit blocks fill less than a wave.  A per call, unsplit / split:

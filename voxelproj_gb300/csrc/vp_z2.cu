@@ -3,14 +3,15 @@
 // In z_order 2 the height axis is the slowest one: x (H, SY, SX) and
 // y (H, n_ang, PX).  The projector's weights do not depend on the height,
 // so the fast kernels put heights across the lanes of a warp; that needs
-// heights contiguous.  For H >= 32 the z_order 2 operators therefore run as
+// heights contiguous.  For H >= 32, and for the forward from 5 heights on where
+// it has the scratch, the z_order 2 operators therefore run as
 //     transpose the input to height-fastest order  (HBM-bound tiled transpose)
 //     z_order 0 kernel, storing (not accumulating) into scratch
 //     transpose the result back, adding it to the caller's output
 // which costs about 2 * (|x| + |y|) of extra HBM traffic, a fraction of a
 // millisecond at 512^3 against several milliseconds of projector work, and
-// keeps the reference's accumulate semantics.  Small H keeps the native
-// z_order 2 kernels (lanes across x / PX).
+// keeps the reference's accumulate semantics.  Other small H run the kernels
+// for few heights (vp_thin.cu: lanes across bins / voxels).
 //
 // Scratch: SY*SX*Hp + n_ang*PX*Hp floats (Hp = H rounded up to 4), supplied by
 // the caller (vp_*_z2_ws) or taken from a library-private stream-ordered pool.
