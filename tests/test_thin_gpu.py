@@ -61,3 +61,20 @@ def test_voxels_outside_a_bin_do_not_reach_it():
     assert not torch.isnan(y).any()
     hit = torch.isinf(y).sum(dim=2)
     assert int(hit.max()) <= 3 and int(hit.min()) >= 1
+
+
+@pytest.mark.parametrize("n", [360, 251])
+@pytest.mark.parametrize("H", [1, 2, 4])
+def test_large_slices_match_many_heights(H, n):
+    """512 x 512 slices at many angles (every rounding of an edge against a tile's border):
+    the thin forward against the transposed path of 8 heights."""
+    g = torch.Generator(device="cuda").manual_seed(9)
+    a = torch.tensor(lin(n, 0.0, 3.1415927), device="cuda")
+    x = torch.randn(8, 512, 500, device="cuda", generator=g)
+    want = torch.zeros(8, n, 520, device="cuda")
+    vp._CU.forward_z2(x, want, a)
+    y = torch.zeros(H, n, 520, device="cuda")
+    vp._CU.forward_z2(x[:H].contiguous(), y, a)
+    # two float32 evaluations of one bin coordinate: the bound of either against 64 bits
+    err = (y - want[:H]).abs().max() / want.abs().max()
+    assert err <= 2 * tol.ref_vs_fp64(520)

@@ -7,10 +7,11 @@
 // with tail(m) the area beyond m >= 0 of the footprint, F(-m) = tail(m),
 //   adjoint, r = round(xp), xv = r - xp:  w0 = tail(1/2 - xv),
 //     w2 = tail(1/2 + xv), w1 = 1 - w0 - w2        (bins r - 1, r + 1, r)
-//   forward, t = |p - xp|:  w = F(1/2 - t) - tail(1/2 + t).
+//   forward: the tails of the voxels that an edge between bins cuts, from
+//     which the weights of the bins on its two sides differ.
 // They are the same piecewise quadratics as trap_cdf (vp_common.cuh), term by
 // term on the side of the footprint where they are needed: about 30
-// instructions for the adjoint's three weights and 15 for one forward weight.
+// instructions for the adjoint's three weights.
 //
 // What bounds them: instruction issue (one slice moves a few MB).
 #include <cuda_runtime.h>
@@ -26,6 +27,7 @@ namespace {
 
 constexpr int kMaxGridYZ = 65535;
 constexpr int THIN_WARPS = 4;
+constexpr int THIN_BINS = 31;  // bins per warp of the forward
 
 // Element strides of the volume and the sinogram: (height, voxel) and
 // (height, bin).
@@ -54,23 +56,25 @@ __device__ __forceinline__ float bin_distance(float fp, float rel_minor, float r
 }
 
 // ---------------------------------------------------------------------------
-// Forward.  A warp owns 32 neighbouring bins of one angle and a quarter of
+// Forward.  A warp owns 31 neighbouring bins of one angle and a quarter of
 // the major lines; the four warps of a block add up their sums in shared
 // memory.  The lines come in chunks of LC: the piece of the volume that the
-// warp's bins see on them (at most 31 sqrt(2) + LC + 6 voxels along the minor
+// warp's bins see on them (at most 31 sqrt(2) + LC + 7 voxels along the minor
 // axis) is read row by row, whichever axis is the minor one, into a shared
-// tile, line-major, and each lane gathers its 3 or 4 voxels per line from
-// there.
+// tile, line-major.  A lane evaluates one edge between bins, which cuts two
+// voxels per line; its bin's other edge comes from the lane below, and with
+// it the bin's four weights.
 //
-// 512 x 512, 360 angles: one slice 1838 -> 320 us, 4 slices 2239 -> 662 us
-// (the kernel before, fp_z2_kernel, took the voxels straight from global
-// memory: 32 cache lines per load where y is the minor axis, one wave of
-// warps that each waited for every line's loads in turn).  One slice issues
-// in 80% of the cycles; its busiest pipe is ALU (70%).
+// 512 x 512, 360 angles: one slice 1838 -> 279 us, 4 slices 2239 -> 564 us
+// (the kernel before took the voxels straight from global memory: 32 cache
+// lines per load where y is the minor axis, one wave of warps that each waited
+// for every line's loads in turn).  With both edges of the bin evaluated for
+// each of its 3 or 4 voxels, on 32 bins per warp: 315 and 594 us.  One slice
+// issues in 80% of the cycles.
 // ---------------------------------------------------------------------------
 template <int LC>
 struct ThinTile {
-  static constexpr int W = (45 + LC + 6) | 1;  // odd pitch: column writes hit all banks
+  static constexpr int W = (45 + LC + 7) | 1;  // odd pitch: column writes hit all banks
 };
 
 // UT elements of the tile: lines l .. l + UT - 1 of voxel m (LINES), or voxels m,
@@ -109,37 +113,49 @@ __device__ __forceinline__ float bin_centre(float q, int i, float cent_major, fl
 }
 
 struct ThinChunk {
-  int i0, nl, m0, nh;  // lines [i0, i0 + nl), the tile's first voxel, heights
+  int i0, nl, m0;  // lines [i0, i0 + nl), the tile's first voxel
   float cent_major, cent_minor, sh_major, inv;
 };
 
-// This lane's bin on the lines of one chunk.  FOUR: 4 voxels per bin and line,
-// else 3.
-template <int RH, int LC, int TRIG, bool MX, bool FOUR>
+// This lane's bin on the lines of one chunk.  fe: the bin's edge on the side of
+// larger minor coordinates; the other edge is that of the lane below.  An edge
+// at minor coordinate u cuts at most the voxels m = floor(u) and m + 1: t0 of
+// the first lies beyond it and t1 of the second before it.  A bin is 1 to 1.42
+// voxels wide, so with m the lower edge's voxel is m - n, n = 1, 2 (or 0 by
+// rounding), and four weights are left.
+template <int RH, int LC, int TRIG, bool MX>
 __device__ __forceinline__ void gather_lines(float (&acc)[RH],
                                              const float (*tl)[LC][ThinTile<LC>::W],
-                                             const ThinChunk& c, float fp, const AngleConst& k,
+                                             const ThinChunk& c, float fe, const AngleConst& k,
                                              float pcent) {
-#pragma unroll 2
-  for (int l = 0; l < c.nl; ++l) {
-    const int i = c.i0 + l;
-    const float u = bin_centre(fp, i, c.cent_major, c.sh_major, c.inv, c.cent_minor, pcent);
-    const int first = (FOUR ? (int)floorf(u) : __float2int_rn(u)) - 1;
-    // (inside the tile but for rounding; one unsigned minimum bounds both sides)
-    const int o = (int)min((unsigned)(first - c.m0), (unsigned)(ThinTile<LC>::W - 4));
-    const float rel_major = (float)i - c.cent_major;
-    const float rel_first = (float)(c.m0 + o) - c.cent_minor;
+  const float sign = c.inv > 0.0f ? 1.0f : -1.0f;
+  const float u0 = bin_centre(fe, c.i0, c.cent_major, c.sh_major, c.inv, c.cent_minor, pcent);
+  const float du = -c.sh_major * c.inv;
+  const float base = (float)(c.m0 + 2) - c.cent_minor;
+  float fl = 0.0f;
+  float rel_major = (float)c.i0 - c.cent_major;
+#pragma unroll 1  // (2 and 4: one slice 283 and 288 us, 1: 279)
+  for (int l = 0; l < c.nl; ++l, fl += 1.0f, rel_major += 1.0f) {
+    // (inside the tile, one voxel of which on either side is for rounding; the
+    // minimum only bounds the index)
+    const int o = (int)min((unsigned)(__float2int_rd(fmaf(fl, du, u0)) - (c.m0 + 2)),
+                           (unsigned)(ThinTile<LC>::W - 4));
+    const float rel = base + (float)o;
+    const float z0 = sign * bin_distance<MX, TRIG>(fe, rel, rel_major, k, pcent);
+    const float z1 = sign * bin_distance<MX, TRIG>(fe, rel + 1.0f, rel_major, k, pcent);
+    const float t0 = tail_area(z0, k), t1 = tail_area(-z1, k);
+    const float s0 = __shfl_up_sync(0xffffffffu, t0, 1);
+    const float s1 = __shfl_up_sync(0xffffffffu, t1, 1);
+    const int n = o - __shfl_up_sync(0xffffffffu, o, 1);
+    const float w[4] = {n >= 2 ? s0 : 0.0f,
+                        n >= 2 ? 1.0f - s1 : n == 1 ? s0 : 0.0f,
+                        (1.0f - t0) - (n >= 2 ? 0.0f : n == 1 ? s1 : 1.0f - s0),
+                        t1 - (n >= 1 ? 0.0f : s1)};
 #pragma unroll
-    for (int t = 0; t < (FOUR ? 4 : 3); ++t) {
-      const float d = fabsf(bin_distance<MX, TRIG>(fp, rel_first + (float)t, rel_major, k, pcent));
-      const float z = 0.5f - d;
-      const float e = __saturatef((k.b - 0.5f) - d);
-      const float f = 0.5f + copysignf(0.5f - tail_area(fabsf(z), k), z);
-      const float w = fmaf(-(k.cd * e), e, f);
-      if (w != 0.0f) {  // (a voxel that the bin does not see adds nothing, whatever it holds)
+    for (int t = 0; t < 4; ++t) {
+      if (w[t] != 0.0f) {  // (a voxel that the bin does not see adds nothing, whatever it holds)
 #pragma unroll
-        for (int h = 0; h < RH; ++h)
-          if (h < c.nh) acc[h] = fmaf(w, tl[h][l][o + t], acc[h]);
+        for (int h = 0; h < RH; ++h) acc[h] = fmaf(w[t], tl[h][l][o + t], acc[h]);
       }
     }
   }
@@ -153,7 +169,6 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
   __shared__ float tile[THIN_WARPS][RH][LC][W];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  const int p = blockIdx.x * 32 + lane;
   const int a = a_base + blockIdx.y;
   const int h0 = blockIdx.z * RH;
   const int nh = min(RH, g.H - h0);
@@ -166,10 +181,10 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
   const float cent_minor = minor_x ? g.xcent : g.ycent;
   const float sh_major = minor_x ? k.s : k.c;
   const float inv = 1.0f / (minor_x ? k.c : k.s);
-  const float fp = (float)p;
-  // a bin's voxels lie within (b + 1/2) |inv| of it along the minor axis: the
-  // nearest three, or the four around it
-  const bool four = (2.0f * k.b + 1.0f) * fabsf(inv) > 2.9f;
+  // lanes 1 .. 31 own bins, in the order of their minor coordinates
+  const int p0 = blockIdx.x * THIN_BINS;
+  const int p = inv > 0.0f ? p0 + lane - 1 : p0 + THIN_BINS - lane;
+  const float fe = (float)p + (inv > 0.0f ? 0.5f : -0.5f);
   const long long s_maj = minor_x ? (long long)g.SX * st.xv : st.xv;
   const long long s_min = minor_x ? st.xv : (long long)g.SX * st.xv;
   const float* xs = x + h0 * st.xh;
@@ -185,10 +200,10 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
 
   for (int i0 = warp * LC; i0 < n_major; i0 += THIN_WARPS * LC) {
     // the chunk's voxels along the minor axis: [m0, m0 + nm)
-    const float q0 = (float)(blockIdx.x * 32), q1 = q0 + 31.0f;
+    const float q0 = (float)p0 - 0.5f, q1 = q0 + (float)THIN_BINS;
     const int i1 = min(i0 + LC, n_major) - 1;
     const float ua = centre(q0, i0), ub = centre(q1, i0), uc = centre(q0, i1), ud = centre(q1, i1);
-    const int m0 = (int)floorf(fminf(fminf(ua, ub), fminf(uc, ud))) - 2;
+    const int m0 = (int)floorf(fminf(fminf(ua, ub), fminf(uc, ud))) - 3;
     const int m1 = min(m0 + W, (int)ceilf(fmaxf(fmaxf(ua, ub), fmaxf(uc, ud))) + 3);
     if (m1 <= 0 || m0 >= n_minor) continue;  // warp-uniform
     const int nl = i1 - i0 + 1;
@@ -209,14 +224,9 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
         tile_load<RH, LC, UT, false>(tl, corner, l, m, nm, l < nl, nh, st.xh, s_maj, s_min, m0, n_minor);
     }
     __syncwarp();
-    const ThinChunk c{i0, nl, m0, nh, cent_major, cent_minor, sh_major, inv};
-    if (minor_x) {
-      if (four) gather_lines<RH, LC, TRIG, true, true>(acc, tl, c, fp, k, g.pcent);
-      else gather_lines<RH, LC, TRIG, true, false>(acc, tl, c, fp, k, g.pcent);
-    } else {
-      if (four) gather_lines<RH, LC, TRIG, false, true>(acc, tl, c, fp, k, g.pcent);
-      else gather_lines<RH, LC, TRIG, false, false>(acc, tl, c, fp, k, g.pcent);
-    }
+    const ThinChunk c{i0, nl, m0, cent_major, cent_minor, sh_major, inv};
+    if (minor_x) gather_lines<RH, LC, TRIG, true>(acc, tl, c, fe, k, g.pcent);
+    else gather_lines<RH, LC, TRIG, false>(acc, tl, c, fe, k, g.pcent);
   }
 
   // the block's four sums
@@ -225,7 +235,7 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
 #pragma unroll
   for (int h = 0; h < RH; ++h) sums[(warp * RH + h) * 32 + lane] = acc[h];
   __syncthreads();
-  if (p >= g.PX) return;
+  if (lane == 0 || p >= g.PX) return;
   for (int h = warp; h < nh; h += THIN_WARPS) {
     float v = 0.0f;
 #pragma unroll
@@ -372,7 +382,7 @@ template <int RH, int LC>
 cudaError_t launch_fp(const float* x, float* y, const float* angles, const Geom& g, int z,
                       cudaStream_t stream) {
   for (int a = 0; a < g.n_ang; a += kMaxGridYZ) {
-    const dim3 grid(ceil_div(g.PX, 32), g.n_ang - a < kMaxGridYZ ? g.n_ang - a : kMaxGridYZ,
+    const dim3 grid(ceil_div(g.PX, THIN_BINS), g.n_ang - a < kMaxGridYZ ? g.n_ang - a : kMaxGridYZ,
                     ceil_div(g.H, RH));
     if (g.trig == TRIG_PRECISE)
       fp_thin_kernel<RH, LC, TRIG_PRECISE><<<grid, 32 * THIN_WARPS, 0, stream>>>(
