@@ -21,7 +21,7 @@ N = 21
 
 @pytest.mark.parametrize("z", [0, 2])
 @pytest.mark.parametrize("Hx,Hy", [(1, 1), (1, 6), (3, 2), (4, 9), (5, 5), (7, 3), (9, 8), (8, 9),
-                                   (31, 31), (33, 33), (45, 47), (130, 129), (203, 203), (257, 260)])
+                                   (31, 31), (33, 33), (45, 47), (130, 129), (203, 203), (257, 260), (300, 290)])
 @pytest.mark.parametrize("SY,SX,PX", [(20, 26, 31), (150, 41, 90)])
 def test_host_heights(SY, SX, PX, Hx, Hy, z):
     H = min(Hx, Hy)

@@ -655,11 +655,11 @@ cudaError_t forward_z0_host(const float* x_host, float* y_host, const float* ang
     float *xd = nullptr, *yd = nullptr, *yc = nullptr, *as = nullptr, *raw = nullptr;
     const float* ad = nullptr;
     Geom gd = g;  // with the device input's heights per row
+    VP_TRY(input_buffer(OP_FORWARD_Z0, g, (size_t)g.SY * g.SX, g.Hx, buf, pool, &xd, &raw,
+                        &gd.Hx));
     VP_TRY(buf.get(pool, y_elems * sizeof(float), &yd));
     if (g.accumulate) VP_TRY(buf.get(pool, y_elems * sizeof(float), &yc));
     VP_TRY(alloc_angles(angles, g, buf, pool, &ad, &as));
-    VP_TRY(input_buffer(OP_FORWARD_Z0, g, (size_t)g.SY * g.SX, g.Hx, buf, pool, &xd, &raw,
-                        &gd.Hx));
     const FwdZ0IO io{x_host, y_host, g, xd, yd, yc, raw, gd.Hx, launches};
     return forward_pipeline(io, angles, gd, xd, yd, as, ad, s, launches);
   }, s);
@@ -676,11 +676,11 @@ cudaError_t backward_z0_host(const float* y_host, float* x_host, const float* an
     float *yd = nullptr, *xd = nullptr, *xc = nullptr, *as = nullptr, *raw = nullptr;
     const float* ad = nullptr;
     Geom gd = g;  // with the device input's heights per row
+    VP_TRY(input_buffer(OP_BACKWARD_Z0, g, (size_t)g.n_ang * g.PX, g.Hy, buf, pool, &yd, &raw,
+                        &gd.Hy));
     VP_TRY(buf.get(pool, x_elems * sizeof(float), &xd));
     if (g.accumulate) VP_TRY(buf.get(pool, x_elems * sizeof(float), &xc));
     VP_TRY(alloc_angles(angles, g, buf, pool, &ad, &as));
-    VP_TRY(input_buffer(OP_BACKWARD_Z0, g, (size_t)g.n_ang * g.PX, g.Hy, buf, pool, &yd, &raw,
-                        &gd.Hy));
     const BwdZ0IO io{y_host, x_host, g, yd, xd, xc, raw, gd.Hy, launches};
     return backward_pipeline(io, angles, gd, yd, xd, as, ad, s, launches);
   }, s);
@@ -719,12 +719,16 @@ cudaError_t z2_backward_chunked(const float* y_host, float* x_host, const float*
     float *in_d[2] = {}, *out_d[2] = {}, *ws[2] = {}, *as = nullptr;
     const float* ad = nullptr;
     const bool pipelined = z2_uses_transpose(gc);
-    const size_t ws_elems = pipelined ? z2_workspace_bytes(gc) / sizeof(float) : 0;
     const int slots = nchunks > 1 ? 2 : 1;
     for (int i = 0; i < slots; ++i) {
-      VP_TRY(buf.get(pool, (size_t)Hc * bins * sizeof(float), &in_d[i]));
-      VP_TRY(buf.get(pool, (size_t)Hc * vox * sizeof(float), &out_d[i]));
-      if (ws_elems > 0) VP_TRY(buf.get(pool, ws_elems * sizeof(float), &ws[i]));
+      // the second slot of two chunks holds the last one only
+      Geom gi = gc;
+      gi.H = gi.Hx = gi.Hy = i == 1 && nchunks == 2 ? H - Hc : Hc;
+      VP_TRY(buf.get(pool, (size_t)gi.H * bins * sizeof(float), &in_d[i]));
+      VP_TRY(buf.get(pool, (size_t)gi.H * vox * sizeof(float), &out_d[i]));
+      if (!pipelined) continue;
+      if (gi.H < 5) gi.H = 5;  // (transposed all the same, in whole float4)
+      VP_TRY(buf.get(pool, z2_workspace_bytes(gi), &ws[i]));
     }
     VP_TRY(alloc_angles(angles, g, buf, pool, &ad, &as));
     auto chunk = [&](int k) {
