@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(32 * BPR_WARPS, R == 8 ? 5 : 0)
   if (yi0 >= row_end || (PASS == 1 && xi0 >= g.SX)) return;
   using Wait = std::conditional_t<PDL, PdlWait, NoWait>;
   bp_runs_warp<PASS, R, Wait, ADD, FULL, VOUT>(y, x, angles, g, xi0, yi0,
-                                         blockIdx.y * 32 * R + lane * 4, accumulate, tab[w],
+                                         blockIdx.y * 32 * R + lane * (R == 2 ? 2 : 4), accumulate, tab[w],
                                          alist[w], Wait(), addend);
 }
 
@@ -543,7 +543,11 @@ cudaError_t launch_bp_z0_runs(const float* y, float* x, const float* angles, con
 }
 
 // Runs with 8 heights per lane on heights [0, r8_heights(H)) and 4 on the
-// rest (one part when H <= 128 or the split leaves no remainder).
+// rest (one part when H <= 128 or the split leaves no remainder).  The default
+// takes a rest of at most 64 heights with 2 per lane: every lane then holds
+// some, half the multiply-adds per window, and the same sums.  A^T with 4 / 2 per
+// lane: (300, 300, 64) and 360 angles 819 / 629 us, (256, 256, 32) and 180 306 /
+// 235, (384, 384, 16) and 180 651 / 497, 64^3 and 128 37 / 35.
 int bp0_split(const Geom& g) { return g.H > 128 ? r8_heights(g.H) : 0; }
 
 cudaError_t launch_bp_z0_runs_split(const float* y, float* x, const float* angles,
@@ -566,6 +570,10 @@ cudaError_t launch_bp_z0_runs_split(const float* y, float* x, const float* angle
   // after the 8-height part's run launches (the bulk-copy form has no
   // programmatic wait, so a launch after it is an ordinary one); the addend
   // wait was taken there, if there was one
+  if (kernel_variant(OP_BACKWARD_Z0) == 0 && g4.H <= 64)
+    return launch_bp_z0_runs<2>(y + H8, x + H8, angles, g4, row_lo, row_hi, stream,
+                                addend ? addend + H8 : nullptr, H8 > 0,
+                                H8 > 0 ? nullptr : addend_ready);
   return launch_bp_z0_runs<4>(y + H8, x + H8, angles, g4, row_lo, row_hi, stream,
                               addend ? addend + H8 : nullptr, H8 > 0 && !tma,
                               H8 > 0 ? nullptr : addend_ready);

@@ -209,7 +209,7 @@ __device__ __forceinline__ void bp_runs_warp(const float* __restrict__ y, float*
                                              const Wait& wait = Wait(),
                                              const float* __restrict__ addend = nullptr) {
   using V = typename Vec<R>::T;
-  static_assert(R == 4 || R == 8, "heights per lane: 4 or 8");
+  static_assert(R == 2 || R == 4 || R == 8, "heights per lane: 2, 4 or 8");
   const int lane = threadIdx.x & 31;
   const LaneH<R> lh(h, g.H);
   const int dx = PASS == 0 ? 1 : 0;

@@ -178,7 +178,13 @@ __device__ __forceinline__ float4 f4_fma(float w, float4 v, float4 acc) {
   return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 
+__device__ __forceinline__ float2 f4_fma(float w, float2 v, float2 acc) {
+  return __ffma2_rn(make_float2(w, w), v, acc);
+}
 __device__ __forceinline__ float f4_fma(float w, float v, float acc) { return fmaf(w, v, acc); }
+__device__ __forceinline__ float2 f4_add(float2 a, float2 b) {
+  return make_float2(a.x + b.x, a.y + b.y);
+}
 
 __device__ __forceinline__ float4 f4_add(float4 a, float4 b) {
   return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
@@ -189,6 +195,8 @@ template <typename T>
 __device__ __forceinline__ T vzero();
 template <>
 __device__ __forceinline__ float vzero<float>() { return 0.0f; }
+template <>
+__device__ __forceinline__ float2 vzero<float2>() { return make_float2(0.f, 0.f); }
 template <>
 __device__ __forceinline__ float4 vzero<float4>() { return make_float4(0.f, 0.f, 0.f, 0.f); }
 
@@ -218,6 +226,10 @@ struct Vec<1> {
   using T = float;
 };
 template <>
+struct Vec<2> {
+  using T = float2;
+};
+template <>
 struct Vec<4> {
   using T = float4;
 };
@@ -226,7 +238,7 @@ struct Vec<8> {
   using T = float4x2;
 };
 
-// Height offsets of one lane: R = 1 or 4 heights from h; R = 8 as float4 at
+// Height offsets of one lane: R = 1, 2 or 4 heights from h; R = 8 as float4 at
 // h and h + 128.  Lanes past H read offset 0 (always valid) and never store.
 template <int R>
 struct LaneH {
@@ -281,6 +293,9 @@ struct Geom {
 __device__ __forceinline__ void store_out(float4* p, float4 v, int accumulate) {
   *p = accumulate ? f4_add(*p, v) : v;
 }
+__device__ __forceinline__ void store_out(float2* p, float2 v, int accumulate) {
+  *p = accumulate ? f4_add(*p, v) : v;
+}
 __device__ __forceinline__ void store_out(float* p, float v, int accumulate) {
   *p = accumulate ? *p + v : v;
 }
@@ -289,6 +304,9 @@ __device__ __forceinline__ void store_out(float* p, float v, int accumulate) {
 // block of the same launch, or the kernel before this one in a programmatic
 // launch, wrote while this block ran, since L1 is not coherent across SMs.
 __device__ __forceinline__ void store_out_coherent(float4* p, float4 v, int accumulate) {
+  *p = accumulate ? f4_add(__ldcg(p), v) : v;
+}
+__device__ __forceinline__ void store_out_coherent(float2* p, float2 v, int accumulate) {
   *p = accumulate ? f4_add(__ldcg(p), v) : v;
 }
 __device__ __forceinline__ void store_out_coherent(float* p, float v, int accumulate) {
@@ -326,7 +344,7 @@ __device__ __forceinline__ void store_lane_heights(float* p, const LaneH<R>& lh,
 #pragma unroll
   for (int k = 0; k < LaneH<R>::NQ; ++k) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < (R < 4 ? R : 4); ++i) {
       const int h = lh.h + k * kSecondHalf + i;
       if (h < H) {
         if constexpr (COHERENT) store_out_coherent(p + h, parts[4 * k + i], accumulate);
