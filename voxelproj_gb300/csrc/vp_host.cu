@@ -508,8 +508,11 @@ cudaError_t backward_pipeline(const IO& io, const float* angles, const Geom& g, 
   // the first sixth of the angles runs over the whole volume first, while
   // the rest of the sinogram arrives (at 512^3 with 192 angles, 12 slabs
   // and a sixth measured 6.22 ms per call; 16 and an eighth 6.37 ms; 8 and
-  // a quarter 6.72 ms)
-  const int a_split = g.n_ang >= 8 ? g.n_ang / 6 : 0;
+  // a quarter 6.72 ms); not for a sinogram of less than 4 MB, which arrives
+  // (20 us) sooner than the extra launches and copies take: (29, 50, 150) and 50
+  // angles 142 with, 120 us without
+  const int a_split = g.n_ang >= 8 && (size_t)g.n_ang * ang_elems >= ((size_t)1 << 20)
+                          ? g.n_ang / 6 : 0;
   HostCtx* c = nullptr;
   VP_TRY(get_ctx(2 * nslabs + 6, &c));
   cudaEvent_t ev_alloc = c->ev[0], ev_in0 = c->ev[1], ev_in = c->ev[2], ev_out = c->ev[3],
