@@ -193,7 +193,7 @@ __device__ __forceinline__ RunEntry run_entry(const float* angles, int a, const 
 }
 
 // One warp: the run of class PASS starting at voxel (xi0, yi0), this lane's
-// heights from h (R = 4: [h, h + 4); R = 8: also [h + 128, h + 132); FULL:
+// heights from h (R = 2, 4: [h, h + R); R = 8: [h, h + 4) and [h + 128, h + 132); FULL:
 // all of them inside [0, H)).  tab
 // (BPR_CHUNK entries) and alist (BPR_LIST ints) are this warp's shared
 // tables.  All 32 lanes must call it together.  wait() runs (by the whole

@@ -109,12 +109,13 @@ cudaError_t pad_heights(const float* src, float* dst, long long rows, int Hs, in
 // that the float4 kernels run (their epilogues write such outputs by single
 // heights).  The copy costs one read and one write of the input; the scalar
 // kernels it replaces held one height per lane: (301, 257, 203) and 181 angles,
-// A 3.76 -> 1.16 ms, A^T 3.00 -> 0.81 ms.  (Up to 32
-// heights the scalar adjoint needs one chunk as well, but at 2 heights per lane
-// the run adjoint is the faster one: 256 x 256, 180 angles 381 against 246 us with 9 heights, 383
-// against 249 with 31.)
+// A 3.76 -> 1.16 ms, A^T 3.00 -> 0.81 ms.  (Up to 32 heights the
+// scalar adjoint needs one chunk as well; it is slower than 2 heights per lane:
+// 256 x 256, 180 angles 381 against 246 us with 9 heights, 383 against 249
+// with 31.)
 inline bool z0_pads(int op, const Geom& g) {
-  return kernel_variant(op) == 0 && !(op == OP_FORWARD_Z0 ? z0_forward_thin(g) : z0_backward_thin(g));
+  return kernel_variant(op) == 0 &&
+         !(op == OP_FORWARD_Z0 ? z0_forward_thin(g) : z0_backward_thin(g));
 }
 
 // z_order 2 through the z_order 0 kernels (vp_z2.cu).
