@@ -109,13 +109,38 @@ cudaError_t pad_heights(const float* src, float* dst, long long rows, int Hs, in
 // that the float4 kernels run (their epilogues write such outputs by single
 // heights).  The copy costs one read and one write of the input; the scalar
 // kernels it replaces held one height per lane: (301, 257, 203) and 181 angles,
-// A 3.76 -> 1.16 ms, A^T 3.00 -> 0.81 ms.  (Up to 32 heights the
-// scalar adjoint needs one chunk as well; it is slower than 2 heights per lane:
-// 256 x 256, 180 angles 381 against 246 us with 9 heights, 383 against 249
-// with 31.)
+// A 3.76 -> 1.16 ms, A^T 3.00 -> 0.81 ms.
+// Few angles do not pay for it.  The adjoint then runs two class launches and
+// the copy where the scalar kernel is one launch, and the 256-height forward
+// has a block for 16 bins (or 4 angles x 4 bins) where the scalar one has 8 by
+// 32-height chunks.  Times by scalar / padded rows, in us:
+//   A^T 512 x 512 x 15: 1 angle 33 / 88, 8 angles 85 / 138, 30 angles 247 / 225;
+//   A^T 128 x 128 x 131: 8 angles 31 / 44, 16 angles 51 / 51;
+//   A^T 64 x 64 x 127: 30 angles 26 / 27, 60 angles 46 / 34;
+//   A^T 24 x 24 x 203: 60 angles 34 / 37, 120 angles 63 / 52;
+//   A 128 x 128 x 203: 16 angles 138 / 185, 30 angles 201 / 174;
+//   A 64 x 64 x 203: 30 angles 67 / 84, 60 angles 110 / 96;
+//   A 512 x 512 x 511, 1 angle: 0.65 / 1.07 ms between synchronisations (the
+//   copy's memory, past what its pool keeps, is mapped anew).
+// Up to 128 heights the banded forward takes 1.2 to 7 times less at any number of
+// angles, the copy included; its 128 + rest parts up to 192 take no more from 4
+// angles or 48 x 48 voxels on.
+inline bool z0_pad_pays(int op, const Geom& g) {
+  const long long vox = (long long)g.SY * g.SX;
+  const int n = g.n_ang;
+  if (op == OP_FORWARD_Z0) {
+    if (g.H <= 192) return g.H <= 128 || n >= 4 || vox >= 48 * 48;
+    if (vox >= 320 * 320) return n >= (g.H <= 256 ? 1 : 8);
+    return n >= (vox >= 192 * 192 ? 16 : vox >= 128 * 128 ? 30 : vox >= 64 * 64 ? 60 : 240);
+  }
+  if (16ll * g.PX > vox) return false;  // (the sinogram is the copy)
+  if (vox < 128 * 128) return n >= (vox < 64 * 64 ? 120 : 60);
+  if (g.H > 32) return n >= 16;
+  return n >= (vox >= 256 * 256 ? 30 : 60);
+}
 inline bool z0_pads(int op, const Geom& g) {
   return kernel_variant(op) == 0 &&
-         !(op == OP_FORWARD_Z0 ? z0_forward_thin(g) : z0_backward_thin(g));
+         !(op == OP_FORWARD_Z0 ? z0_forward_thin(g) : z0_backward_thin(g)) && z0_pad_pays(op, g);
 }
 
 // z_order 2 through the z_order 0 kernels (vp_z2.cu).
