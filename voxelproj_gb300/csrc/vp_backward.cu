@@ -275,8 +275,8 @@ __global__ void __launch_bounds__(TMA_THREADS, 4)
 }
 
 // ---------------------------------------------------------------------------
-// z_order 2 in the reference's order of additions (with variant 4), below 32
-// heights: x (H, SY, SX), y (H, n_ang, PX); x / PX are contiguous.
+// z_order 2 below 32 heights, in the reference's order of additions (variant 4,
+// and few angles: launch_backward_z2): x (H, SY, SX), y (H, n_ang, PX); x / PX are contiguous.
 // A thread owns one voxel column (lane <-> xi, so loads and stores coalesce
 // along x) and BP2_RH heights.  Weights are per thread (lanes hold different
 // voxels) and are reused across the thread's heights.  Angle constants for a
@@ -661,8 +661,14 @@ cudaError_t launch_backward_z0_rows_add(const float* y, float* x, const float* a
 
 cudaError_t launch_backward_z2(const float* y, float* x, const float* angles, const Geom& g,
                                cudaStream_t stream) {
-  // (the reference's order of additions goes with the z_order 0 variant that has it)
-  if (kernel_variant(OP_BACKWARD_Z0) != 4)
+  // bp_z2_kernel has the reference's order of additions (it goes with the z_order
+  // 0 variant that has it), and is the faster one for fewer than 8 angles where
+  // its blocks fill about a wave at most: 128 x 128 x 16 and 1 angle 6.4 us, the
+  // kernel for few heights 8.3; 256 x 256 x 8 and 2 angles the same, but 384 x 384
+  // x 16 and 4 angles 17 and 13
+  const bool small = g.n_ang < 8 && g.H > 4 &&
+                     (long long)g.SY * g.SX * ceil_div(g.H, BP2_RH) <= 160000;
+  if (kernel_variant(OP_BACKWARD_Z0) != 4 && !small)
     return launch_backward_thin(y, x, angles, g, 2, stream);
   dim3 block(32, BP2_WARPS);
   dim3 grid(ceil_div(g.SX, 32), ceil_div(g.SY, BP2_WARPS), ceil_div(g.H, BP2_RH));

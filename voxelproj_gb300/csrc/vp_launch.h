@@ -99,7 +99,12 @@ int launches_forward_thin(const Geom& g);
 // 582 -> 200 (8), but 583 -> 545 (16) and 477 -> 529 (19); A^T 363 -> 39 (1),
 // 367 -> 67 (3), 378 -> 107 (7), but 321 -> 644 (16).
 inline bool z0_forward_thin(const Geom& g) { return g.H <= 4; }
-inline bool z0_backward_thin(const Geom& g) { return g.H <= 7 && g.H % 4 != 0; }
+// (Of 5 to 7 heights, small volumes with fewer than 8 angles stay on the scalar
+// kernel: 24 x 24 x 7, 4 angles 8 us, 10 on this one.)
+inline bool z0_backward_thin(const Geom& g) {
+  if (g.n_ang < 8 && g.H > 4 && (long long)g.SY * g.SX < 32 * 32) return false;
+  return g.H <= 7 && g.H % 4 != 0;
+}
 
 // dst rows of Hd floats from src rows of Hs: heights [0, H), then zeros; dst
 // 16-byte aligned, Hd a multiple of 4 (vp_z2.cu).

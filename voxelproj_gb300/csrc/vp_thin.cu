@@ -246,12 +246,14 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
 
 // ---------------------------------------------------------------------------
 // Adjoint.  A lane owns VR voxels, neighbours along y, of 32 columns; the
-// angles' constants come from a per-warp shared table, 32 angles at a time.
-// With SPLIT the four warps of a block take the same voxels and a quarter of
-// the angles each and add up in shared memory (small volumes: enough warps to
+// angles' constants come from a per-warp shared table, at most 32 angles at a
+// time.  With SPLIT the four warps of a block take the same voxels and a quarter
+// of the angles each and add up in shared memory (small volumes: enough warps to
 // fill the GPU); else neighbouring rows.  Z2: bins are contiguous, else heights.
 // 512 x 512, 360 angles: one slice 304 -> 137 us, 8 slices 932 -> 554 us.  One
-// slice issues in 75% of the cycles.
+// slice issues in 75% of the cycles.  With tables of 32 angles whatever their
+// number, the first warp had all of up to 32 angles: 256 x 256 x 8 and 30 angles
+// 83 us, 24 with equal shares; 24 x 24 x 16 58 and 14.
 // ---------------------------------------------------------------------------
 template <int RH, int VR, bool SPLIT, bool Z2, int TRIG>
 __global__ void __launch_bounds__(32 * THIN_WARPS)
@@ -278,15 +280,19 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
 #pragma unroll
     for (int h = 0; h < RH; ++h) acc[v][h] = 0.0f;
 
-  const int step = SPLIT ? 32 * THIN_WARPS : 32;
-  for (int a0 = SPLIT ? 32 * warp : 0; a0 < g.n_ang; a0 += step) {
+  // angles per table: with SPLIT as many as give the four warps equal shares
+  constexpr int kMost = 32 * (SPLIT ? THIN_WARPS : 1);
+  const int rounds = (g.n_ang + kMost - 1) / kMost;
+  const int at = SPLIT ? (g.n_ang + rounds * THIN_WARPS - 1) / (rounds * THIN_WARPS) : 32;
+  const int step = SPLIT ? at * THIN_WARPS : 32;
+  for (int a0 = SPLIT ? at * warp : 0; a0 < g.n_ang; a0 += step) {
     __syncwarp();
-    if (a0 + lane < g.n_ang) {
+    if (lane < at && a0 + lane < g.n_ang) {
       const AngleConst k = angle_const(__ldg(angles + a0 + lane), TRIG);
       tab[warp][lane] = Entry{make_float4(k.a, k.b, k.coeff, k.cd), make_float2(k.c, k.s)};
     }
     __syncwarp();
-    const int na = min(32, g.n_ang - a0);
+    const int na = min(at, g.n_ang - a0);
     const float* ya = y + h0 * yh + (long long)a0 * g.PX * yb;
     for (int j = 0; j < na; ++j, ya += g.PX * yb) {
       const Entry& e = tab[warp][j];
@@ -397,7 +403,8 @@ cudaError_t launch_fp(const float* x, float* y, const float* angles, const Geom&
 }
 
 // Blocks of 4 warps below which the adjoint splits the angles over them
-// (152 SMs, about 12 resident blocks each).
+// (152 SMs, about 12 resident blocks each).  From 8 angles on: with fewer a
+// quarter of them saves less than the sum over the warps costs.
 constexpr long long kSplitRows = 4096;
 constexpr long long kFourVoxels = 4096;  // rows of 32 voxels per slice
 
@@ -407,7 +414,7 @@ cudaError_t launch_bp(const float* y, float* x, const float* angles, const Geom&
   const long long rows = ceil_div(g.SY, VR);
   const long long warps = (long long)ceil_div(g.SX, 32) * rows * ceil_div(g.H, RH);
   const ThinStrides st = thin_strides(g, z);
-  const bool split = warps < kSplitRows && rows <= kMaxGridYZ;
+  const bool split = warps < kSplitRows && rows <= kMaxGridYZ && g.n_ang >= 2 * THIN_WARPS;
   const dim3 grid(ceil_div(g.SX, 32), split ? (unsigned)rows : ceil_div(rows, THIN_WARPS),
                   ceil_div(g.H, RH));
   const auto kernel = g.trig == TRIG_PRECISE
@@ -424,8 +431,9 @@ cudaError_t launch_bp_z(const float* y, float* x, const float* angles, const Geo
                         cudaStream_t stream) {
   // four voxels per lane share an angle's constants where that leaves enough
   // warps; 512 x 512, 360 angles: one slice 209 us with one, 177 with two, 152
-  // with four; 64 x 64, 60 angles: 12 us with one, 20 with four
-  const bool four = (long long)ceil_div(g.SX, 32) * g.SY >= kFourVoxels;
+  // with four; 64 x 64, 60 angles: 12 us with one, 20 with four; 384 x 384 x 4 and
+  // 2 angles 10.4 with one, 13.7 with four
+  const bool four = (long long)ceil_div(g.SX, 32) * g.SY >= kFourVoxels && g.n_ang >= 8;
   if (g.H == 1)
     return four ? launch_bp<1, 4, Z2>(y, x, angles, g, z, stream)
                 : launch_bp<1, 1, Z2>(y, x, angles, g, z, stream);
