@@ -193,6 +193,28 @@ __device__ __forceinline__ BandAngle band_angle(const AngleConst& k, const Geom&
   return A;
 }
 
+// Cuts [lo, hi) to the lines on which a window of the G runs from run0 can meet
+// the slab's voxels; the others add nothing.  On line i bin q has its centre at
+// minor coordinate c(q) - s (i - cent_major); 3 voxels are kept beyond the
+// windows, far above the rounding of either side.
+// Where the detector is wider than the volume, or the volume longer than broad,
+// many runs see few lines: A (40, 300, 48) with 240 angles and 450 bins 460 us
+// with all lines, candidate lists 287, 168 with this.
+template <int G>
+__device__ __forceinline__ void band_clip(const BandAngle& A, const Geom& g, int run0, int* lo,
+                                          int* hi) {
+  constexpr float kBelow = (float)Band<false>::W + 3.0f, kAbove = (float)Band<false>::before + 3.0f;
+  const float s = A.sh_major * A.inv;
+  if (!(fabsf(s) > 1e-6f)) return;  // no line differs from the next (or NaN)
+  const float qa = (float)(4 * run0), qb = qa + (float)(4 * G - 1);
+  const float ca = (qa - g.pcent) * A.inv + A.cent_minor, cb = (qb - g.pcent) * A.inv + A.cent_minor;
+  const float u = (fmaxf(ca, cb) - ((float)A.min_lo - kBelow)) / s;
+  const float v = (fminf(ca, cb) - ((float)A.min_hi + kAbove)) / s;
+  const float first = floorf(fminf(u, v) + A.cent_major), last = ceilf(fmaxf(u, v) + A.cent_major);
+  *lo = max(*lo, (int)fmaxf(first, -1.0f));
+  *hi = max(*lo, (int)fminf((float)*hi, last + 1.0f));
+}
+
 // The sums of G runs from run0 on share `part` of SP of the slab's lines.
 template <int G, int SP>
 __device__ __forceinline__ void band_sums(float4 (&acc)[4], const float* xs, const BandAngle& A,
@@ -203,6 +225,7 @@ __device__ __forceinline__ void band_sums(float4 (&acc)[4], const float* xs, con
     lo = min(lo + part * share, hi);
     hi = min(lo + share, hi);
   }
+  band_clip<G>(A, g, run0, &lo, &hi);
   if ((2.0f * A.k.b + 1.0f) * fabsf(A.inv) <= kBandNarrow)
     band_lines<G, true>(acc, xs, A, g, run0, lo, hi, tab);
   else
