@@ -177,9 +177,9 @@ struct Fp0Config {
 // per block, the volume staged through shared memory by tensor copies
 // (vp_fp_staged.cuh); 19 = the aligned angle groups with plain loads; 21 /
 // 22 / 23 = as 16 with 128 / 32 / 256 MB slabs.  The default (0) is 16 with
-// 8 heights per lane; at most 128 heights, and a rest of 129 to 192 in two
-// parts, run the banded 4-height form (vp_fp_band.cuh), at most 4 heights the
-// kernel of vp_thin.cu.  Measured A per call with programmatic launches between the slab
+// 8 heights per lane; at most 128 heights (also as the rest past 256), and 129 to
+// 192 in two parts where that pays (fp0_parts_pay), run the banded 4-height form
+// (vp_fp_band.cuh), at most 4 heights the kernel of vp_thin.cu.  Measured A per call with programmatic launches between the slab
 // launches, variants 16 / 21 / 22 / 23: 512^3 and 192 angles 6.66 / 6.73 /
 // 7.05 / 7.12 ms; 1024 angles 32.98 / 33.89 / 35.06 ms; 256^3 and 360 angles
 // 1.534 / 1.585 / 1.551 ms; 384^3 and 641 angles 10.54 / 10.50 / 11.01 ms.
@@ -513,38 +513,45 @@ cudaError_t launch_fp_z0_config(const float* x, float* y, const float* angles, c
 }
 
 // The heights of a call as (first height, count) parts: one part, or with 8
-// heights per lane an 8-height part and 4-height parts for the rest
-// (r8_heights).  The default's banded 4-height form also takes a rest of 129 to
-// 192 heights, as 128 and what is left: about 46 + 27 clocks per SM, line and
-// run of bins against 76 for a whole 256-height chunk.
+// heights per lane an 8-height part and a 4-height part for the rest
+// (r8_heights).  The default's banded 4-height form also takes 129 to 192 heights,
+// as 128 and what is left.
 struct HeightParts {
   int n;
-  Geom g[3];
-  int h0[3];
+  Geom g[2];
+  int h0[2];
 };
 
+// Whether 129 to 192 heights take less as two banded parts than in the 256-height
+// form.  That form has one block for 16 bins and 256 heights, so below a wave of
+// its blocks (7 per SM) the two parts fill more of the GPU; from there on they pay
+// while the second part leaves lanes of no warp idle (at most 32 heights, 4 runs
+// per warp).  A in us, 256-height form / parts: 128 x 128 x 180 and 100 angles 190 /
+// 145, 400 angles 462 / 501; 256 x 256 x 180 and 30 angles 201 / 185, 200 angles
+// 889 / 977; 256 x 256 x 144 and 200 angles 866 / 689; 32 x 32 x 144 and 400
+// angles 47 / 49, 160 heights 47 / 53.  More than 256 heights stay in that form:
+// 64 x 64 x 416 and 100 angles 95 against 128 in three parts, 512 x 512 x 416 and
+// 30 1387 against 1330.
+bool fp0_parts_pay(const Geom& g) {
+  const long long blocks = (long long)ceil_div(g.PX, 4) * ceil_div(g.n_ang, FP0_WARPS);
+  const long long vox = (long long)g.SY * g.SX;
+  return blocks <= (vox >= 64 * 64 ? 7 * 152 : 512) || (g.H <= 160 && vox >= 48 * 48);
+}
+
 HeightParts fp0_parts(const Geom& g, bool vec4, int variant) {
-  HeightParts p{0, {g, g, g}, {0, 0, 0}};
+  HeightParts p{0, {g, g}, {0, 0}};
   const auto add = [&](int h0, int H) {
     p.h0[p.n] = h0;
     p.g[p.n].H = H;
     ++p.n;
   };
-  if (fp0_config(g, vec4, variant).R != 8) {
-    add(0, g.H);
-    return p;
+  int first = g.H;
+  if (fp0_config(g, vec4, variant).R == 8) {
+    first = r8_heights(g.H);
+    if (variant == 0 && g.H > 128 && g.H <= 192 && fp0_band_ok(g) && fp0_parts_pay(g)) first = 128;
   }
-  int H8 = r8_heights(g.H);
-  const int full = g.H / 256 * 256, rest = g.H - full;
-  if (variant == 0 && fp0_band_ok(g) && rest > 128 && rest <= 192) {
-    H8 = full;
-    if (full > 0) add(0, full);
-    add(full, 128);
-    if (rest > 128) add(full + 128, rest - 128);
-    return p;
-  }
-  if (H8 > 0) add(0, H8);
-  if (H8 < g.H) add(H8, g.H - H8);
+  if (first > 0) add(0, first);
+  if (first < g.H) add(first, g.H - first);
   return p;
 }
 
