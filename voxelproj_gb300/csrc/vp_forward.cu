@@ -189,22 +189,43 @@ struct Fp0Config {
 // the same bin layout (the default gets them padded: z0_pads); 8-height
 // variants on problems of at most 128 heights run the 4-height form.
 
-// Whether the banded 4-height form splits a run's lines over four warps: when
-// its unsplit blocks fill less than a wave.  A per call, unsplit / split:
-// 32^3 and 128 angles (64 blocks) 16.5 / 8.3 us; 64^3 and 128 (256 blocks)
-// 28.8 / 22.6; 256 x 256 x 12 and 180 (360) 173 / 121; 384 x 384 x 16 and 180
-// (540) 273 / 243; 128^3 and 192 (1536 blocks, 1.7 waves) 147 / 147; 96^3 and
-// 300 (1800) 124 / 131.  Without a device to ask, no.
-bool fp0_band_split(const Geom& g, int runs_per_warp) {
+// SMs of the current device; 0 without one to ask.
+int fp0_sms() {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      sms <= 0) {
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return 0;
   }
-  const double blocks = (double)ceil_div(g.PX, 4 * runs_per_warp * FP0_WARPS) * g.n_ang;
-  return blocks < 6.0 * sms;  // 5 or 6 resident blocks per SM
+  return sms;
+}
+
+// The default's 4-height form is banded, with the fewest lanes per run that hold
+// the heights.  Its run's lines are split over four warps (split) while its unsplit
+// blocks fill less than a wave of 6 per SM, for sides above 64 up to 16 per SM, and
+// with one run per warp up to 12: split blocks are a quarter as long and level the
+// SMs better, at the price of one more weight table pass per warp where the lines
+// of a share fill no table.  A in us, unsplit / split: 32^3 and 128 angles (64 blocks)
+// 16.5 / 8.3; 384 x 384 x 16 and 180 (540) 273 / 243; 128^3 and 125 (1000) 130 / 103,
+// 312 (2496) 241 / 231, 1000 (8000) 682 / 703; 256 x 256 x 16 and 150 (300) 148 / 106.
+// Volumes of at most 48 x 48 stay on the candidate lists (band 0) above 64 heights
+// and from 3 blocks per SM on, where neither form gains on them (24 x 24 x 100 and
+// 375 angles: lists 22.9, banded 23.1, split 25.1), with two warps per run where twice as many
+// half-long blocks take fewer half-waves of 8 per SM or fill less than three
+// quarters of one.  Without a device to ask, no split.
+void fp0_narrow_config(const Geom& g, Fp0Config* c) {
+  const int sms = fp0_sms();
+  const int side = g.SY > g.SX ? g.SY : g.SX;
+  const int runs = fp0_band_runs(g.H);
+  const double blocks = (double)ceil_div(g.PX, 4 * runs * FP0_WARPS) * g.n_ang;
+  if (runs == 1 && side <= 48 && blocks >= 3.0 * sms) {
+    const double w = blocks / (8.0 * (sms > 0 ? sms : 1));
+    c->split = sms > 0 && w < 2.0 && (std::ceil(2.0 * w) < 2.0 * std::ceil(w) || w <= 0.75);
+    return;
+  }
+  c->band = runs;
+  c->split = blocks < 6.0 * sms || (side > 64 && blocks < 16.0 * sms) ||
+             (runs == 1 && blocks < 12.0 * sms);
 }
 
 Fp0Config fp0_config(const Geom& g, bool vec4, int variant) {
@@ -238,15 +259,9 @@ Fp0Config fp0_config(const Geom& g, bool vec4, int variant) {
     c.R = vec4 ? 4 : 1;
     c.un = FP0_UNROLL;
     c.staged = 0;
-    // the default's 4-height form is banded, with the fewest lanes per run that
-    // hold the heights, and splits a run's lines over four warps when its
-    // blocks fill less than one wave
     if (dflt) {
       c.agroup = false;
-      if (vec4 && fp0_band_ok(g)) {
-        c.band = fp0_band_runs(g.H);
-        c.split = fp0_band_split(g, c.band);
-      }
+      if (vec4 && fp0_band_ok(g)) fp0_narrow_config(g, &c);
     }
   }
   return c;
@@ -293,6 +308,17 @@ Slab fp0_slab(const Geom& g, const Fp0Config& c, int k, int n) {
   int wy = 0, wx = 0;
   fp0_slab_widths(g, c, n, &wy, &wx);
   return slab_of(k, c.cls, wy, wx, g.SY, g.SX);
+}
+
+// Lines per partial sum of the banded form (vp_fp_band.cuh): at most kBandLines, and no
+// more than a slab of 256-height chunks has.
+int fp0_band_lines(const Geom& g) {
+  Fp0Config c = fp0_config(g, false, 16);
+  c.R = 8;
+  int wy = 0, wx = 0;
+  fp0_slab_widths(g, c, fp0_slabs(g, c), &wy, &wx);
+  const int w = wy > wx ? wy : wx;
+  return w < kBandLines ? w : kBandLines;
 }
 
 // Rows of x take float4 loads; rows of y float4 stores.
@@ -460,7 +486,7 @@ cudaError_t launch_slab_aligned(const SlabLaunch& L, cudaStream_t stream, int* l
 cudaError_t launch_slab_config(const Fp0Config& c, const SlabLaunch& L, cudaStream_t s, int* n) {
   if (c.band)
     return launch_fp_band(BandLaunch{L.x, L.y, L.angles, L.g, L.slab, L.accumulate, L.a_lo, L.a_hi,
-                                     L.programmatic, L.vec_out},
+                                     L.programmatic, L.vec_out, fp0_band_lines(L.g)},
                           c.band, c.split, s, n);
   if (!L.vec_out && c.R != 1) {  // the default's forms (fp0_vec4)
     if (c.R == 8) return launch_slab<8, 4, true, 2, false, false, false>(L, s, n);

@@ -24,12 +24,9 @@ template <int G, int SP, bool PDL, bool VOUT>
 __global__ void __launch_bounds__(32 * FPB_WARPS, G == 1 ? 6 : 5)
     fp_band_kernel(const float* __restrict__ x, float* __restrict__ y,
                    const float* __restrict__ angles, Geom g, int a_base, Slab slab,
-                   int accumulate) {
-  union Smem {
-    BandSmem warp[FPB_WARPS];
-    float4 sums[SP > 1 ? FPB_WARPS : 1][32][4];
-  };
-  __shared__ Smem sm;
+                   int accumulate, int lines) {
+  __shared__ BandSmem sm[FPB_WARPS];
+  __shared__ float4 sums[SP > 1 ? FPB_WARPS : 1][32][4];
   pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -39,7 +36,8 @@ __global__ void __launch_bounds__(32 * FPB_WARPS, G == 1 ? 6 : 5)
   const bool has = a < g.n_ang && 4 * G * set < g.PX;
   using Wait = std::conditional_t<PDL, PdlWait, NoWait>;
   fp_band_block<G, SP, Wait, VOUT>(x, y, angles, g, set * G, a, h, slab, has,
-                                   SP > 1 ? warp % SP : 0, accumulate, &sm.warp[warp], sm.sums);
+                                   SP > 1 ? warp % SP : 0, lines, accumulate,
+                                   &sm[warp], sums);
 }
 
 inline unsigned ceil_div(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
@@ -56,9 +54,9 @@ cudaError_t launch_band(const BandLaunch& L, cudaStream_t stream, int* launches)
     const bool p = L.programmatic || a > L.a_lo;
     cudaError_t e =
         p ? launch_ex(fp_band_kernel<G, SP, true, VOUT>, grid, block, 0, stream, true, L.x, L.y,
-                      L.angles, g, (int)a, L.slab, L.accumulate)
+                      L.angles, g, (int)a, L.slab, L.accumulate, L.lines)
           : launch_ex(fp_band_kernel<G, SP, false, VOUT>, grid, block, 0, stream, false, L.x, L.y,
-                      L.angles, g, (int)a, L.slab, L.accumulate);
+                      L.angles, g, (int)a, L.slab, L.accumulate, L.lines);
     if (launches) ++*launches;
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return e;

@@ -211,42 +211,43 @@ __device__ __forceinline__ void band_clip(const BandAngle& A, const Geom& g, int
   const float u = (fmaxf(ca, cb) - ((float)A.min_lo - kBelow)) / s;
   const float v = (fminf(ca, cb) - ((float)A.min_hi + kAbove)) / s;
   const float first = floorf(fminf(u, v) + A.cent_major), last = ceilf(fmaxf(u, v) + A.cent_major);
-  *lo = max(*lo, (int)fmaxf(first, -1.0f));
+  *lo = min(max(*lo, (int)fmaxf(first, -1.0f)), *hi);
   *hi = max(*lo, (int)fminf((float)*hi, last + 1.0f));
 }
 
-// The sums of G runs from run0 on share `part` of SP of the slab's lines.
-template <int G, int SP>
+// The sums of G runs from run0 on the lines [lo, hi).
+template <int G>
 __device__ __forceinline__ void band_sums(float4 (&acc)[4], const float* xs, const BandAngle& A,
-                                          const Geom& g, int run0, int part, BandEntry* tab) {
-  int lo = A.maj_lo, hi = A.maj_hi;
-  if (SP > 1) {
-    const int share = (hi - lo + SP - 1) / SP;
-    lo = min(lo + part * share, hi);
-    hi = min(lo + share, hi);
-  }
-  band_clip<G>(A, g, run0, &lo, &hi);
+                                          const Geom& g, int run0, int lo, int hi,
+                                          BandEntry* tab) {
+#pragma unroll
+  for (int b = 0; b < 4; ++b) acc[b] = vzero<float4>();
   if ((2.0f * A.k.b + 1.0f) * fabsf(A.inv) <= kBandNarrow)
     band_lines<G, true>(acc, xs, A, g, run0, lo, hi, tab);
   else
     band_lines<G, false>(acc, xs, A, g, run0, lo, hi, tab);
 }
 
-// Adds or stores the sums of G runs from run0 on, by the whole warp, after
-// wait(); h: this lane's heights (several runs: of the one chunk).
+// Adds or stores the sums of G runs from run0 on (over the lines [lo, hi)), by the
+// whole warp, after wait(); h: this lane's heights (several runs: of the one
+// chunk).
 template <int G, class Wait, bool VOUT>
 __device__ __forceinline__ void band_write(const float4 (&acc)[4], const float* x, float* y,
                                            const float* angles, const Geom& g, const Slab& s,
-                                           const BandAngle& A, int run0, int a, int h,
-                                           int accumulate, float4* cand, const Wait& wait) {
+                                           const BandAngle& A, int lo, int hi, int run0, int a,
+                                           int h, int accumulate, float4* cand,
+                                           const Wait& wait) {
   wait();
-  if (A.maj_lo >= A.maj_hi && accumulate) return;
+  if (lo >= hi && accumulate) return;
   const int lane = threadIdx.x & 31;
   if (__any_sync(0xffffffffu, not_finite(acc, g.H - h))) {
+    Slab part = s;
+    (A.minor_x ? part.y_lo : part.x_lo) = lo;
+    (A.minor_x ? part.y_hi : part.x_hi) = hi;
     for (int r = 0; r < G; ++r) {
       __syncwarp();
       fp_z0_warp<4, 4, 2, Wait, false, VOUT>(x, y, angles, g, 4 * (run0 + r), a,
-                                             G > 1 ? 4 * lane : h, s, accumulate, cand, wait);
+                                             G > 1 ? 4 * lane : h, part, accumulate, cand, wait);
     }
     return;
   }
@@ -266,47 +267,73 @@ __device__ __forceinline__ void band_write(const float4 (&acc)[4], const float* 
 // Block body.  A warp takes G runs of 4 bins (from run0) of angle a and its
 // lanes' heights from h, on the slab's lines; with SP warps per run set, warp
 // `part` takes every SP-th share of the lines and part 0 writes the sum of all
-// (sums: FPB_WARPS x 32 x 4 vectors of shared memory).  has: this warp has
-// work (all warps of a block must call).
+// (sums: FPB_WARPS x 32 x 4 vectors of shared memory, where partial sums of
+// `lines` lines gather too; with one warp they are added into y).  has: this warp
+// has work (all warps of a block must call, with SP = 4 with the same runs).
 template <int G, int SP, class Wait, bool VOUT>
 __device__ __forceinline__ void fp_band_block(const float* __restrict__ x, float* __restrict__ y,
                                               const float* __restrict__ angles, const Geom& g,
                                               int run0, int a, int h, const Slab& s, bool has,
-                                              int part, int accumulate, BandSmem* sm,
+                                              int part, int lines, int accumulate, BandSmem* sm,
                                               float4 (*sums)[32][4]) {
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const Wait wait;
-  float4 acc[4];
-#pragma unroll
-  for (int b = 0; b < 4; ++b) acc[b] = vzero<float4>();
-  BandAngle A;
-  if (has) {
-    A = band_angle(angle_const(__ldg(angles + a), g.trig), g, s);
-    band_sums<G, SP>(acc, x + (h < g.H ? h : 0), A, g, run0, part, sm->tab);
-  }
-  if (SP > 1) {
-    __syncthreads();
-    if (part > 0)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) sums[warp][lane][b] = acc[b];
-    __syncthreads();
-    if (part == 0) {
-#pragma unroll
-      for (int j = 1; j < SP; ++j)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[b] = f4_add(acc[b], sums[warp + j][lane][b]);
-      __syncwarp();
-    }
-  }
-  if (!has || part > 0) {
+  if (!has) {  // (with SP = 4: the whole block)
     wait();
     return;
   }
-  band_write<G, Wait, VOUT>(acc, x, y, angles, g, s, A, run0, a, h, accumulate, sm->cand, wait);
+  const float* xs = x + (h < g.H ? h : 0);
+  float4 acc[4];
+  const BandAngle A = band_angle(angle_const(__ldg(angles + a), g.trig), g, s);
+  int lo = A.maj_lo, hi = A.maj_hi;
+  band_clip<G>(A, g, run0, &lo, &hi);
+  if constexpr (SP == 1) {
+    for (;;) {
+      const int end = min(lo + lines, hi);
+      band_sums<G>(acc, xs, A, g, run0, lo, end, sm->tab);
+      band_write<G, Wait, VOUT>(acc, x, y, angles, g, s, A, lo, end, run0, a, h, accumulate,
+                                sm->cand, wait);
+      if (end >= hi) return;
+      lo = end;
+      accumulate = 1;
+    }
+  } else {
+    const int all_lo = lo, all_hi = hi, share = (hi - lo + SP - 1) / SP;
+    lo = min(lo + part * share, hi);
+    hi = min(lo + share, hi);
+    float4* mine = sums[warp][lane];
+    for (bool first = true;; first = false) {
+      const int end = min(lo + lines, hi);
+      band_sums<G>(acc, xs, A, g, run0, lo, end, sm->tab);
+      if (!first) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[b] = f4_add(mine[b], acc[b]);
+      }
+      if (end >= hi) break;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) mine[b] = acc[b];
+      lo = end;
+    }
+    if (part > 0)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) mine[b] = acc[b];
+    __syncthreads();
+    if (part > 0) {
+      wait();
+      return;
+    }
+#pragma unroll
+    for (int j = 1; j < SP; ++j)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) acc[b] = f4_add(acc[b], sums[warp + j][lane][b]);
+    band_write<G, Wait, VOUT>(acc, x, y, angles, g, s, A, all_lo, all_hi, run0, a, h, accumulate,
+                              sm->cand, wait);
+  }
 }
 
-// One warp of a batch: as fp_band_block without a split.
+// One warp of a batch: as fp_band_block without a split, in one sum (a batch's
+// slabs are those of the candidate lists).
 template <int G, class Wait>
 __device__ __forceinline__ void fp_band_warp(const float* __restrict__ x, float* __restrict__ y,
                                              const float* __restrict__ angles, const Geom& g,
@@ -317,12 +344,12 @@ __device__ __forceinline__ void fp_band_warp(const float* __restrict__ x, float*
     return;
   }
   float4 acc[4];
-#pragma unroll
-  for (int b = 0; b < 4; ++b) acc[b] = vzero<float4>();
   const BandAngle A = band_angle(angle_const(__ldg(angles + a), g.trig), g, s);
-  band_sums<G, 1>(acc, x + (h < g.H ? h : 0), A, g, run0, 0, sm->tab);
+  int lo = A.maj_lo, hi = A.maj_hi;
+  band_clip<G>(A, g, run0, &lo, &hi);
+  band_sums<G>(acc, x + (h < g.H ? h : 0), A, g, run0, lo, hi, sm->tab);
   __syncwarp();
-  band_write<G, Wait, true>(acc, x, y, angles, g, s, A, run0, a, h, 1, sm->cand, wait);
+  band_write<G, Wait, true>(acc, x, y, angles, g, s, A, lo, hi, run0, a, h, 1, sm->cand, wait);
 }
 
 }  // namespace detail
