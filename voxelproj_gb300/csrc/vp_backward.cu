@@ -547,7 +547,10 @@ cudaError_t launch_bp_z0_runs(const float* y, float* x, const float* angles, con
 // takes a rest of at most 64 heights with 2 per lane: every lane then holds
 // some, half the multiply-adds per window, and the same sums.  A^T with 4 / 2 per
 // lane: (300, 300, 64) and 360 angles 819 / 629 us, (256, 256, 32) and 180 306 /
-// 235, (384, 384, 16) and 180 651 / 497, 64^3 and 128 37 / 35.
+// 235, (384, 384, 16) and 180 651 / 497, 64^3 and 128 37 / 35.  A rest past 256
+// heights does so from 128 x 128 voxels on: in smaller volumes its launches, which
+// overlap the 8-height ones, take longer with 2: (72, 72, 300) and 120 angles 74 / 99,
+// (128, 128, 300) 174 / 177, (160, 160, 300) 259 / 246.
 int bp0_split(const Geom& g) { return g.H > 128 ? r8_heights(g.H) : 0; }
 
 cudaError_t launch_bp_z0_runs_split(const float* y, float* x, const float* angles,
@@ -570,7 +573,8 @@ cudaError_t launch_bp_z0_runs_split(const float* y, float* x, const float* angle
   // after the 8-height part's run launches (the bulk-copy form has no
   // programmatic wait, so a launch after it is an ordinary one); the addend
   // wait was taken there, if there was one
-  if (kernel_variant(OP_BACKWARD_Z0) == 0 && g4.H <= 64)
+  const bool small_rest = H8 > 0 && (long long)g.SY * g.SX < 128 * 128;
+  if (kernel_variant(OP_BACKWARD_Z0) == 0 && g4.H <= 64 && !small_rest)
     return launch_bp_z0_runs<2>(y + H8, x + H8, angles, g4, row_lo, row_hi, stream,
                                 addend ? addend + H8 : nullptr, H8 > 0,
                                 H8 > 0 ? nullptr : addend_ready);
