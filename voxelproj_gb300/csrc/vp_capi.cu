@@ -71,6 +71,17 @@ cudaMemPool_t g_pools[kMaxDevices] = {};
 constexpr uint64_t kPadPoolKeep = (uint64_t)256 << 20;
 cudaMemPool_t g_pad_pools[kMaxDevices] = {};
 
+// While it lives, this thread's pool calls leave stream captures of other threads
+// alone (making a pool, taking memory from it and giving it back would invalidate a
+// capture in the global mode; none of them touches a capturing stream here).
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  RelaxedCapture(const RelaxedCapture&) = delete;
+  RelaxedCapture& operator=(const RelaxedCapture&) = delete;
+};
+
 cudaError_t device_pool(cudaMemPool_t (&pools)[kMaxDevices], uint64_t keep, cudaMemPool_t* out) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -178,11 +189,11 @@ cudaError_t padded_input(int op, const float* in, int64_t rows, int Hin, const v
   if (e != cudaSuccess) return e;
   if (cap != cudaStreamCaptureStatusNone) return cudaSuccess;
   cudaMemPool_t pool;
-  if ((e = device_pool(g_pad_pools, kPadPoolKeep, &pool)) != cudaSuccess) return e;
   *Hp = (g.H + 3) / 4 * 4;
   void* p = nullptr;
-  if (cudaMallocFromPoolAsync(&p, (size_t)rows * *Hp * sizeof(float), pool, stream) !=
-      cudaSuccess) {
+  if (device_pool(g_pad_pools, kPadPoolKeep, &pool) != cudaSuccess ||
+      cudaMallocFromPoolAsync(&p, (size_t)rows * *Hp * sizeof(float), pool, stream) !=
+          cudaSuccess) {
     cudaGetLastError();  // no room: run on the input itself
     return cudaSuccess;
   }
@@ -201,6 +212,7 @@ int run_z0(bool forward, const float* in, float* out, const float* angles, vp::G
   const int64_t rows = forward ? (int64_t)g.SY * g.SX : (int64_t)g.n_ang * g.PX;
   float* copy = nullptr;
   int Hp = 0;
+  const RelaxedCapture relaxed;
   cudaError_t e =
       padded_input(op, in, rows, forward ? g.Hx : g.Hy, g, stream, &copy, &Hp);
   if (e != cudaSuccess) return finish(e, 0);
@@ -357,6 +369,7 @@ int run_z2(bool forward, const float* in, float* out, const float* angles, const
     use = false;
   }
   bool owned = false;
+  const RelaxedCapture relaxed;
   if (use && ws == nullptr) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (!must) {
