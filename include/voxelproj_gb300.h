@@ -179,11 +179,11 @@ VP_API int vp_project_store(int op, int z_order, const float* in, const int64_t 
  * (64 MiB) compiled into the library, held by every GPU that loads the
  * library until the process exits.  Problems of 32 heights or more that need
  * more scratch than that (vp_z2_workspace_bytes) return VP_ERR_SCRATCH_LIMIT and
- * leave y unchanged; with fewer heights they run without scratch.
- * The first call on a device looks up the array's address (make it before
- * any stream capture).  All calls share the array: calls that overlap on the
- * GPU race and must be ordered by the caller.  No counterpart in the
- * reference. */
+ * leave y unchanged.  The first such call on a device looks up the array's
+ * address (make it before any stream capture).  All calls of 32 heights or more
+ * share the array: those that overlap on the GPU race and must be ordered by the
+ * caller.  Below 32 heights a kernel without scratch runs: such calls may overlap,
+ * be captured first, and be of any size.  No counterpart in the reference. */
 #define VP_NOALLOC_SCRATCH_BYTES ((size_t)64 << 20)
 VP_API int vp_forward_z2_noalloc(const float* x, int64_t x0, int64_t x1, int64_t x2,
                                  float* y, int64_t y0, int64_t y1, int64_t y2,

@@ -523,13 +523,13 @@ extern "C" int vp_project_store(int op, int z_order, const float* in, const int6
 // cudaGetSymbolAddress, with that device current, and caches it.  Make that
 // first call before any stream capture.
 //
-// All calls on a device share the array, and it keeps whatever the previous
-// call left.  Nothing in this path reads scratch before writing it: the
-// input is transposed into the array, the projector stores (not adds) its
-// result there, and only those values are copied back.  Pad heights up to a
-// multiple of 4 carry leftovers, but they are never copied out.  Two calls
-// that overlap on the GPU (different streams, no ordering between them) race
-// on the array and corrupt each other's results.
+// All calls of 32 heights or more on a device share the array, and it keeps
+// whatever the previous call left.  Nothing in this path reads scratch before
+// writing it: the input is transposed into the array (pad heights up to a multiple
+// of 4 as zeros), the projector stores (not adds) its result there, and only the
+// heights of the problem are copied back.  Two calls that overlap on the GPU
+// (different streams, no ordering between them) race on the array and corrupt each
+// other's results.
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -566,13 +566,15 @@ extern "C" int vp_forward_z2_noalloc(const float* x, int64_t x0, int64_t x1, int
   if (int s = make_geom(x, x1, x2, x0, y, y1, y2, y0, angles, n_angles, flags, &g, &empty))
     return s;
   if (empty) return VP_OK;
-  const size_t need = vp::z2_workspace_bytes(g);
-  // (below 32 heights a problem past the array runs without scratch)
-  if (need > VP_NOALLOC_SCRATCH_BYTES && vp::z2_uses_transpose(g)) return VP_ERR_SCRATCH_LIMIT;
-  float* scratch = nullptr;
-  if (need > 0) {
-    const cudaError_t e = noalloc_scratch(&scratch);
-    if (e != cudaSuccess) return finish(e, 0);
+  // Below 32 heights the kernel for few heights runs, which needs no scratch: such
+  // calls may overlap, and may be a device's first under stream capture.
+  if (!vp::z2_uses_transpose(g)) {
+    const cudaError_t e = vp::launch_forward_thin(x, y, angles, g, 2, (cudaStream_t)stream);
+    return finish(e, vp::launches_forward_thin(g));
   }
+  if (vp::z2_workspace_bytes(g) > VP_NOALLOC_SCRATCH_BYTES) return VP_ERR_SCRATCH_LIMIT;
+  float* scratch = nullptr;
+  const cudaError_t e = noalloc_scratch(&scratch);
+  if (e != cudaSuccess) return finish(e, 0);
   return run_z2(true, x, y, angles, g, scratch, VP_NOALLOC_SCRATCH_BYTES, (cudaStream_t)stream);
 }
