@@ -146,7 +146,7 @@ VP_API int vp_backward_z2(const float* y, int64_t y0, int64_t y1, int64_t y2,
  * transpose back (adding into the output); they need
  * vp_z2_workspace_bytes(...) bytes of device scratch.  From 5 to 31
  * heights the forward does so too where it gets the scratch, and runs without
- * it otherwise; below 5 heights the size is 0.  The
+ * it otherwise (the adjoint uses none there); below 5 heights the size is 0.  The
  * plain vp_forward_z2 / vp_backward_z2 take it from a library-private
  * stream-ordered pool; these variants use `workspace` instead and fail with
  * VP_ERR_WORKSPACE if it is too small for 32 heights or more.  No counterpart in the reference,

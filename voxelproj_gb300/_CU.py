@@ -76,13 +76,25 @@ except AttributeError:  # pragma: no cover
         return torch.cuda.current_stream(index).cuda_stream
 
 
+_Z2_SCRATCH_HEIGHTS = 32  # z_order 2 cannot do without its scratch from here on
+
+
 def _z2_workspace(inp, out, forward: bool):
-    """Scratch for the transposed path from torch's caching allocator, or None."""
+    """Scratch for the transposed path from torch's caching allocator, or None:
+    with fewer heights the adjoint uses none, and the forward runs without it
+    where there is no memory for it."""
     x, y = (inp, out) if forward else (out, inp)
+    optional = min(x.shape[0], y.shape[0]) < _Z2_SCRATCH_HEIGHTS
     nbytes = _lib.LIB.vp_z2_workspace_bytes(*x.shape, *y.shape)
-    if not nbytes:
+    if not nbytes or (optional and not forward):
         return None, 0
-    return torch.empty((nbytes + 3) // 4, dtype=torch.float32, device=inp.device), nbytes
+    try:
+        ws = torch.empty((nbytes + 3) // 4, dtype=torch.float32, device=inp.device)
+    except torch.cuda.OutOfMemoryError:
+        if not optional:
+            raise
+        return None, 0
+    return ws, nbytes
 
 
 def _on_device(device, fn):
