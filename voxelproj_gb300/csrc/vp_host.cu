@@ -624,25 +624,24 @@ cudaError_t z0_thin_host(bool forward, const float* in_host, float* out_host,
   }, s);
 }
 
-// The device buffer of a pipeline's input: rows x Hin floats, or, where the
-// float4 kernels want padded rows (z0_pads) and there is memory for both, rows x
-// Hp with *raw to arrive in.
-cudaError_t input_buffer(int op, const Geom& g, size_t rows, int Hin, Buffers& buf,
-                         cudaMemPool_t pool, float** dev, float** raw, int* Hp) {
+// A second device buffer for a pipeline's input of rows x Hin floats at *dev, where
+// the float4 kernels want padded rows (z0_pads) and there is memory left: rows x Hp
+// at *dev then, and the input arrives at *raw.  Taken after every buffer that the
+// call cannot do without.
+void pad_buffer(int op, const Geom& g, size_t rows, int Hin, Buffers& buf, cudaMemPool_t pool,
+                float** dev, float** raw, int* Hp) {
   *raw = nullptr;
   *Hp = Hin;
-  VP_TRY(buf.get(pool, rows * Hin * sizeof(float), dev));
-  if (Hin % 4 == 0 || !z0_pads(op, g)) return cudaSuccess;
+  if (Hin % 4 == 0 || !z0_pads(op, g)) return;
   float* padded = nullptr;
   const int hp = (g.H + 3) / 4 * 4;
   if (buf.get(pool, rows * hp * sizeof(float), &padded) != cudaSuccess) {
     cudaGetLastError();  // no room: run on the input itself
-    return cudaSuccess;
+    return;
   }
   *raw = *dev;
   *dev = padded;
   *Hp = hp;
-  return cudaSuccess;
 }
 
 }  // namespace
@@ -652,17 +651,17 @@ cudaError_t forward_z0_host(const float* x_host, float* y_host, const float* ang
   std::lock_guard<std::mutex> lock(g_mutex);
   if (kernel_variant(OP_FORWARD_Z0) == 0 && z0_forward_thin(g))
     return z0_thin_host(true, x_host, y_host, angles, g, pool, s, launches);
-  const size_t y_elems = (size_t)g.n_ang * g.PX * g.Hy;
+  const size_t x_elems = (size_t)g.SY * g.SX * g.Hx, y_elems = (size_t)g.n_ang * g.PX * g.Hy;
   Buffers buf(s);
   return guarded([&]() -> cudaError_t {
     float *xd = nullptr, *yd = nullptr, *yc = nullptr, *as = nullptr, *raw = nullptr;
     const float* ad = nullptr;
     Geom gd = g;  // with the device input's heights per row
-    VP_TRY(input_buffer(OP_FORWARD_Z0, g, (size_t)g.SY * g.SX, g.Hx, buf, pool, &xd, &raw,
-                        &gd.Hx));
+    VP_TRY(buf.get(pool, x_elems * sizeof(float), &xd));
     VP_TRY(buf.get(pool, y_elems * sizeof(float), &yd));
     if (g.accumulate) VP_TRY(buf.get(pool, y_elems * sizeof(float), &yc));
     VP_TRY(alloc_angles(angles, g, buf, pool, &ad, &as));
+    pad_buffer(OP_FORWARD_Z0, g, (size_t)g.SY * g.SX, g.Hx, buf, pool, &xd, &raw, &gd.Hx);
     const FwdZ0IO io{x_host, y_host, g, xd, yd, yc, raw, gd.Hx, launches};
     return forward_pipeline(io, angles, gd, xd, yd, as, ad, s, launches);
   }, s);
@@ -673,17 +672,17 @@ cudaError_t backward_z0_host(const float* y_host, float* x_host, const float* an
   std::lock_guard<std::mutex> lock(g_mutex);
   if (kernel_variant(OP_BACKWARD_Z0) == 0 && z0_backward_thin(g))
     return z0_thin_host(false, y_host, x_host, angles, g, pool, s, launches);
-  const size_t x_elems = (size_t)g.SY * g.SX * g.Hx;
+  const size_t x_elems = (size_t)g.SY * g.SX * g.Hx, y_elems = (size_t)g.n_ang * g.PX * g.Hy;
   Buffers buf(s);
   return guarded([&]() -> cudaError_t {
     float *yd = nullptr, *xd = nullptr, *xc = nullptr, *as = nullptr, *raw = nullptr;
     const float* ad = nullptr;
     Geom gd = g;  // with the device input's heights per row
-    VP_TRY(input_buffer(OP_BACKWARD_Z0, g, (size_t)g.n_ang * g.PX, g.Hy, buf, pool, &yd, &raw,
-                        &gd.Hy));
+    VP_TRY(buf.get(pool, y_elems * sizeof(float), &yd));
     VP_TRY(buf.get(pool, x_elems * sizeof(float), &xd));
     if (g.accumulate) VP_TRY(buf.get(pool, x_elems * sizeof(float), &xc));
     VP_TRY(alloc_angles(angles, g, buf, pool, &ad, &as));
+    pad_buffer(OP_BACKWARD_Z0, g, (size_t)g.n_ang * g.PX, g.Hy, buf, pool, &yd, &raw, &gd.Hy);
     const BwdZ0IO io{y_host, x_host, g, yd, xd, xc, raw, gd.Hy, launches};
     return backward_pipeline(io, angles, gd, yd, xd, as, ad, s, launches);
   }, s);
@@ -923,11 +922,13 @@ cudaError_t z2_host(bool forward, const float* in_host, float* out_host, const f
                                s));
       else
         VP_TRY(cudaMemsetAsync(ys, 0, (size_t)H * bins * sizeof(float), s));
-      if (z2_can_transpose(gk)) {
-        VP_TRY(buf.get(pool, z2_workspace_bytes(gk), &ws));
+      // (without room for the workspace: the kernel for few heights)
+      if (z2_can_transpose(gk) &&
+          buf.get(pool, z2_workspace_bytes(gk), &ws) == cudaSuccess) {
         VP_TRY(forward_z2_transposed(xs, ys, ad, gk, ws, s));
         *launches += launches_z2(gk, true);
       } else {
+        cudaGetLastError();
         VP_TRY(launch_forward_thin(xs, ys, ad, gk, 2, s));
         *launches += launches_forward_thin(gk);
       }
