@@ -688,12 +688,26 @@ cudaError_t backward_z0_host(const float* y_host, float* x_host, const float* an
   }, s);
 }
 
+// Heights per chunk of the z_order 2 adjoint with host arrays: 256 (the
+// 8-heights-per-lane kernels' chunk) above 256 heights, halves from 129, one chunk up
+// to 128, which the 4-height kernels project at once: (256, 256, 101) and 360 angles
+// 1.10 against 1.76 ms in halves, (384, 384, 300) and 300 4.07 against 5.07.  With few
+// angles the copies take most of a large call, and equal halves (from 65 to 511
+// heights) overlap more of them: (420, 420, 100) and 30 angles 0.80 against 0.91 ms,
+// (512, 512, 257) 2.58 against 3.01, with 60 2.70 against 3.09.
+int z2_adjoint_chunk(const Geom& g) {
+  const int half = ((g.H + 1) / 2 + 3) / 4 * 4;
+  const long long vox = (long long)g.SY * g.SX;
+  const bool copies = g.H <= 128 ? g.n_ang < 75 && vox >= 300 * 300
+                                  : g.n_ang < 100 && vox >= 200 * 200;
+  if (g.H >= 512 || (g.H > 256 && !copies)) return 256;
+  if (g.H > 128 || (g.H > 64 && copies)) return half;
+  return g.H;
+}
+
 // The z_order 2 adjoint with host arrays, by chunks of heights, whose
-// sinogram and volume blocks are contiguous: chunks of 256 heights (the
-// 8-heights-per-lane kernels' chunk) above 256 heights, halves from 129, one
-// chunk up to 128, which the 4-height kernels project at once: (256, 256, 101)
-// and 360 angles 1.10 against 1.76 ms in halves, (384, 384, 300) and 300 4.07
-// against 5.07.  With the transposed path (32 heights and more):
+// sinogram and volume blocks are contiguous (z2_adjoint_chunk).  With the
+// transposed path (32 heights and more):
 //   copy stream:  the chunks' sinograms in order, each container after the
 //                 next chunk's sinogram (a projection needs only its input)
 //   kernel streams (alternating by chunk, one projection at a time): the
@@ -703,16 +717,14 @@ cudaError_t backward_z0_host(const float* y_host, float* x_host, const float* an
 //                 transpose-add into the container and the copy home; the
 //                 last chunk slab by slab, so that most of it is home when
 //                 the kernels end
-// Small heights run the native z_order 2 kernel per chunk on one stream.
+// Small heights run the kernel for them on one stream.
 // Called under g_mutex.
 cudaError_t z2_backward_chunked(const float* y_host, float* x_host, const float* angles,
                                 const Geom& g, cudaMemPool_t pool, cudaStream_t s,
                                 int* launches) {
   const size_t vox = (size_t)g.SY * g.SX, bins = (size_t)g.n_ang * g.PX;
   const int H = g.H;
-  int Hc = H;
-  if (H > 256) Hc = 256;
-  else if (H > 128) Hc = ((H + 1) / 2 + 3) / 4 * 4;
+  const int Hc = z2_adjoint_chunk(g);
   const int nchunks = (H + Hc - 1) / Hc;
   Geom gc = g;  // a full chunk
   gc.H = gc.Hx = gc.Hy = Hc;
