@@ -624,15 +624,28 @@ cudaError_t z0_thin_host(bool forward, const float* in_host, float* out_host,
   }, s);
 }
 
+// Whether a pipeline pads its input's rows (z0_pads: whether a device call does).  The
+// pipelines run by pieces, which fill less of the GPU in the 256-height forward than
+// in the scalar form, and wait for the copies with few angles: A (512, 512, 203) and
+// 8 angles 1.97 ms on the input itself, 2.34 on padded rows; (128, 128, 257) and 30
+// 0.475 / 0.586, 120 angles 0.86 / 0.64; (64, 64, 257) and 120 0.326 / 0.354, 360
+// 0.63 / 0.41.
+bool host_pads(int op, const Geom& g) {
+  if (!z0_pads(op, g)) return false;
+  if (op != OP_FORWARD_Z0 || g.H <= 192) return true;
+  const long long vox = (long long)g.SY * g.SX;
+  return g.n_ang >= (vox >= 192 * 192 ? 30 : vox >= 100 * 100 ? 100 : 240);
+}
+
 // A second device buffer for a pipeline's input of rows x Hin floats at *dev, where
-// the float4 kernels want padded rows (z0_pads) and there is memory left: rows x Hp
+// the float4 kernels want padded rows (host_pads) and there is memory left: rows x Hp
 // at *dev then, and the input arrives at *raw.  Taken after every buffer that the
 // call cannot do without.
 void pad_buffer(int op, const Geom& g, size_t rows, int Hin, Buffers& buf, cudaMemPool_t pool,
                 float** dev, float** raw, int* Hp) {
   *raw = nullptr;
   *Hp = Hin;
-  if (Hin % 4 == 0 || !z0_pads(op, g)) return;
+  if (Hin % 4 == 0 || !host_pads(op, g)) return;
   float* padded = nullptr;
   const int hp = (g.H + 3) / 4 * 4;
   if (buf.get(pool, rows * hp * sizeof(float), &padded) != cudaSuccess) {
