@@ -551,7 +551,9 @@ int part_desc(const vp_batch_problem& p, const vp::Geom& g, const float* in, flo
 // The problem's descriptors: one per height part.  With 8 heights per lane a
 // last chunk of at most 128 heights is a second part with 4 per lane, as in
 // the single-problem launchers (r8_heights).
-int batch_desc(const vp_batch_problem& p, std::vector<vp::BatchDesc>* out) {
+// bands: the default's forwards of 129 to 192 heights go as banded 4-height parts
+// (parts_pay).
+int batch_desc(const vp_batch_problem& p, bool bands, std::vector<vp::BatchDesc>* out) {
   if (p.op != VP_OP_FORWARD && p.op != VP_OP_BACKWARD) return VP_ERR_BATCH;
   if (p.flags & ~VP_FLAG_TRIG_PRECISE) return VP_ERR_BAD_FLAGS;
   const bool fwd = p.op == VP_OP_FORWARD;
@@ -596,17 +598,28 @@ int batch_desc(const vp_batch_problem& p, std::vector<vp::BatchDesc>* out) {
     if (st == VP_OK) out->push_back(d);
     return st;
   };
-  // the default's forward takes a last chunk of 129 to 192 heights by banded
-  // 4-height parts, as the single-problem default does (fp0_parts)
-  const int full = H8 / 256 * 256, rest = H8 - full;
-  if (fwd && p.variant == 0 && R == 8 && rest > 128 && rest <= 192 && vp::fp0_band_ok(g)) {
-    if (full > 0)
-      if (int st = add(0, full, 0)) return st;
-    if (int st = add(full, 128, H8)) return st;
-    return add(full + 128, rest - 128, H8);
+  if (fwd && p.variant == 0 && bands && H > 128 && H <= 192 && vp::fp0_band_ok(g)) {
+    if (int st = add(0, 128, H8)) return st;
+    return add(128, g.H - 128, H8);
   }
   if (int st = add(0, H8, 0)) return st;
   return H8 < g.H ? add(H8, g.H - H8, 0) : VP_OK;
+}
+
+// Whether a batch takes its default forwards of 129 to 192 heights as two banded parts:
+// where no other forward then needs the 8-height body.  Bodies run one after another,
+// so a second one leaves more of the GPU idle than the parts save: eight uneven
+// problems with forwards of 132, 136, 220 and 236 heights 644 us without, 712 with; 3
+// of (40, 40, 400) and 30 angles 67 / 98 (the rest past 256 in parts); but 4 of
+// (160, 160, 160) and 120 angles 948 / 763, 3 of (256, 256, 192) and 200 2732 / 2354.
+bool parts_pay(const vp_batch_problem* problems, int count) {
+  for (int i = 0; i < count; ++i) {
+    const vp_batch_problem& p = problems[i];
+    if (p.op != VP_OP_FORWARD) continue;
+    const int64_t H = p.in_dims[2] < p.out_dims[2] ? p.in_dims[2] : p.out_dims[2];
+    if (H > (p.variant == 0 ? 192 : 128)) return false;
+  }
+  return true;
 }
 
 // A plan's descriptors and bookkeeping for a set of problems: descriptors
@@ -649,9 +662,10 @@ cudaError_t blocks_per_sm(int device, int (&per_sm)[vp::NBODIES], int* sms) {
 int make_layout(const vp_batch_problem* problems, int count, Layout* L) {
   std::vector<vp::BatchDesc> by_body[vp::NBODIES];
   std::vector<vp::BatchDesc> parts;
+  const bool bands = parts_pay(problems, count);
   for (int i = 0; i < count; ++i) {
     parts.clear();
-    if (int s = batch_desc(problems[i], &parts)) return s;
+    if (int s = batch_desc(problems[i], bands, &parts)) return s;
     for (const vp::BatchDesc& d : parts) by_body[vp::body_of(d)].push_back(d);
   }
   L->descs.reserve(2 * (size_t)count);
