@@ -190,6 +190,9 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
   const float* xs = x + h0 * st.xh;
   float(*tl)[LC][W] = tile[warp];
 
+  // each chunk of lines in a sum of its own: an accumulator that runs over a quarter of
+  // all lines had 1.2 times the error of the slabs' sums before it (A (500, 512, 4),
+  // 50 angles, precise)
   float acc[RH];
 #pragma unroll
   for (int h = 0; h < RH; ++h) acc[h] = 0.0f;
@@ -225,8 +228,13 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
     }
     __syncwarp();
     const ThinChunk c{i0, nl, m0, cent_major, cent_minor, sh_major, inv};
-    if (minor_x) gather_lines<RH, LC, TRIG, true>(acc, tl, c, fe, k, g.pcent);
-    else gather_lines<RH, LC, TRIG, false>(acc, tl, c, fe, k, g.pcent);
+    float part[RH];
+#pragma unroll
+    for (int h = 0; h < RH; ++h) part[h] = 0.0f;
+    if (minor_x) gather_lines<RH, LC, TRIG, true>(part, tl, c, fe, k, g.pcent);
+    else gather_lines<RH, LC, TRIG, false>(part, tl, c, fe, k, g.pcent);
+#pragma unroll
+    for (int h = 0; h < RH; ++h) acc[h] += part[h];
   }
 
   // the block's four sums
