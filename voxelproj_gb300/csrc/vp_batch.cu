@@ -583,6 +583,7 @@ int batch_desc(const vp_batch_problem& p, bool bands, std::vector<vp::BatchDesc>
   g.pcent = 0.5f * (float)(g.PX - 1);
   g.trig = (p.flags & VP_FLAG_TRIG_PRECISE) ? vp::TRIG_PRECISE : vp::TRIG_REF;
   g.accumulate = 1;
+  g.skip_zero = 0;
   // heights per lane of the first part
   int R = 4;
   if (fwd)

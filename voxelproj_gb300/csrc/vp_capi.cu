@@ -55,6 +55,7 @@ int make_geom(const void* xp, int64_t SY, int64_t SX, int64_t Hx, const void* yp
   g->pcent = 0.5f * (float)(PX - 1);
   g->trig = (flags & VP_FLAG_TRIG_PRECISE) ? vp::TRIG_PRECISE : vp::TRIG_REF;
   g->accumulate = 1;
+  g->skip_zero = 0;
   return VP_OK;
 }
 
@@ -363,7 +364,7 @@ int run_z2(bool forward, const float* in, float* out, const float* angles, const
            void* ws, size_t ws_bytes, cudaStream_t stream) {
   const size_t need = vp::z2_workspace_bytes(g);
   const bool must = vp::z2_uses_transpose(g);
-  bool use = must || (forward && vp::z2_can_transpose(g));
+  bool use = must || (forward && vp::z2_few_transposes(g));
   if (use && ws != nullptr && ws_bytes < need) {
     if (must) return VP_ERR_WORKSPACE;
     use = false;

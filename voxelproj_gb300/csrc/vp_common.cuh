@@ -287,6 +287,8 @@ struct Geom {
   float xcent, ycent, pcent;
   int trig;
   int accumulate;   // 1: out += result (the reference's semantics); 0: out = result
+  int skip_zero;    // 1: a bin gets nothing from a voxel of weight zero, whatever that
+                    // holds (z_order 2 below 32 heights; finite voxels: no difference)
 };
 
 // Epilogue: out (+)= acc.

@@ -21,7 +21,7 @@
 // (vp_fp_z0.cuh) with the same weights, so the sums are equal bit for bit.
 // A zero weight times an infinite voxel would spread it to bins that do not
 // see it: a warp whose sums are not all finite repeats its runs with the
-// candidate lists.
+// candidate lists (without their zero weights where g.skip_zero).
 #pragma once
 
 #include "vp_common.cuh"
@@ -246,8 +246,9 @@ __device__ __forceinline__ void band_write(const float4 (&acc)[4], const float* 
     (A.minor_x ? part.y_hi : part.x_hi) = hi;
     for (int r = 0; r < G; ++r) {
       __syncwarp();
-      fp_z0_warp<4, 4, 2, Wait, false, VOUT>(x, y, angles, g, 4 * (run0 + r), a,
-                                             G > 1 ? 4 * lane : h, part, accumulate, cand, wait);
+      fp_z0_warp<4, 4, 2, Wait, false, VOUT, true>(x, y, angles, g, 4 * (run0 + r), a,
+                                                   G > 1 ? 4 * lane : h, part, accumulate, cand,
+                                                   wait);
     }
     return;
   }

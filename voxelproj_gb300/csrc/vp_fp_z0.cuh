@@ -107,6 +107,19 @@ __device__ __forceinline__ void scatter_q(V (&acc)[KW], const float4& e, const V
 #undef VP_Q_CASE
 }
 
+// The same without a switch, leaving out zero weights if `skip`: for voxels that are
+// not finite.
+template <int KW, class V>
+__device__ __forceinline__ void scatter_nonzero(V (&acc)[KW], const float4& e, const V& xv, int q,
+                                                bool skip) {
+#pragma unroll
+  for (int b = 0; b < KW; ++b) {
+    const int d = q - b;  // the run's bin b is the voxel's bin 2 - d
+    const float w = d == 2 ? e.x : d == 1 ? e.y : e.z;
+    if (d >= 0 && d <= 2 && !(skip && w == 0.0f)) acc[b] = f4_fma(w, xv, acc[b]);
+  }
+}
+
 // The part of the volume one launch (or one batch stage) gathers from.
 // Angles whose minor axis is x walk rows [y_lo, y_hi) (all columns); angles
 // whose minor axis is y walk columns [x_lo, x_hi) within rows [yy_lo, yy_hi).
@@ -144,8 +157,9 @@ __host__ __device__ inline Slab slab_of(int k, bool cls, int wy, int wx, int SY,
 // Fp0Cap<KW>::list entries.  All 32 lanes must call it together.
 // wait() runs (by the whole warp) just before the outputs are written; with
 // Wait::coherent the read of the output bypasses L1.
+// SKIP: the form that heeds g.skip_zero.
 template <int R, int KW, int UN = FP0_UNROLL, class Wait = NoWait, bool FULL = false,
-          bool VOUT = true>
+          bool VOUT = true, bool SKIP = false>
 __device__ __forceinline__ void fp_z0_warp(const float* __restrict__ x, float* __restrict__ y,
                                            const float* __restrict__ angles, const Geom& g,
                                            int p0, int a, int h, const Slab& s,
@@ -232,7 +246,9 @@ __device__ __forceinline__ void fp_z0_warp(const float* __restrict__ x, float* _
 #pragma unroll
       for (int u = 0; u < UN; ++u) {
         if (c0 + u >= total) break;  // padding slots (warp-uniform)
-        scatter_q<KW>(acc, e[u], xv[u], __float_as_int(e[u].w) & ((1 << FP0_QBITS) - 1));
+        const int q = __float_as_int(e[u].w) & ((1 << FP0_QBITS) - 1);
+        if constexpr (SKIP) scatter_nonzero<KW>(acc, e[u], xv[u], q, g.skip_zero != 0);
+        else scatter_q<KW>(acc, e[u], xv[u], q);
       }
     }
     __syncwarp();

@@ -948,7 +948,7 @@ cudaError_t z2_host(bool forward, const float* in_host, float* out_host, const f
       else
         VP_TRY(cudaMemsetAsync(ys, 0, (size_t)H * bins * sizeof(float), s));
       // (without room for the workspace: the kernel for few heights)
-      if (z2_can_transpose(gk) &&
+      if (z2_few_transposes(gk) &&
           buf.get(pool, z2_workspace_bytes(gk), &ws) == cudaSuccess) {
         VP_TRY(forward_z2_transposed(xs, ys, ad, gk, ws, s));
         *launches += launches_z2(gk, true);

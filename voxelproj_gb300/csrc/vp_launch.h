@@ -160,9 +160,12 @@ inline bool z0_pads(int op, const Geom& g) {
 // From 32 heights on always; from 5 on the forward does where it has the
 // workspace (z2_workspace_bytes, more than 0 then), else it runs the kernel
 // for few heights, which needs none: 384 x 384 x 16, 180 angles 685 against
-// 262 us with the transposes, 512 x 512 x 4 and 360 662 against 780 us.
+// 262 us with the transposes, 512 x 512 x 4 and 360 662 against 780 us.  It does so
+// with the banded form only, which leaves out zero weights as that kernel does
+// (z2_few_transposes).
 bool z2_uses_transpose(const Geom& g);
 bool z2_can_transpose(const Geom& g);
+bool z2_few_transposes(const Geom& g);
 size_t z2_workspace_bytes(const Geom& g);
 int launches_z2(const Geom& g, bool forward);  // of the transposed form
 cudaError_t forward_z2_transposed(const float* x, float* y, const float* angles, const Geom& g,

@@ -189,6 +189,10 @@ bool z2_uses_transpose(const Geom& g) { return g.H >= 32; }
 
 bool z2_can_transpose(const Geom& g) { return g.H >= 5; }
 
+bool z2_few_transposes(const Geom& g) {
+  return z2_can_transpose(g) && kernel_variant(OP_FORWARD_Z0) == 0 && fp0_band_ok(g);
+}
+
 size_t z2_workspace_bytes(const Geom& g) {
   if (!z2_can_transpose(g)) return 0;
   const long long Hp = round4(g.H);
@@ -219,6 +223,8 @@ cudaError_t z2_project(bool forward, const float* in, const float* angles, const
   Geom g0 = g;
   g0.H = g0.Hx = g0.Hy = (int)Hp;
   g0.accumulate = 0;
+  // as the kernel for few heights (vp_thin.cu) does
+  g0.skip_zero = forward && !z2_uses_transpose(g);
   if (forward) {
     const cudaError_t e = transpose(in, xt, g.H, nvox, nvox, Hp, 0, stream, Hp);
     if (e != cudaSuccess) return e;
