@@ -508,11 +508,8 @@ cudaError_t backward_pipeline(const IO& io, const float* angles, const Geom& g, 
   // the first sixth of the angles runs over the whole volume first, while
   // the rest of the sinogram arrives (at 512^3 with 192 angles, 12 slabs
   // and a sixth measured 6.22 ms per call; 16 and an eighth 6.37 ms; 8 and
-  // a quarter 6.72 ms).  A sinogram of less than 4 MB arrives in one piece (20 us),
-  // sooner than the extra copy takes; its angles stay two sums, as of larger ones
-  // ((29, 50, 150) and 50 angles 97 us, in one sum 94 with up to 3% more error).
+  // a quarter 6.72 ms)
   const int a_split = g.n_ang >= 8 ? g.n_ang / 6 : 0;
-  const bool pieces = a_split > 0 && (size_t)g.n_ang * ang_elems >= ((size_t)1 << 20);
   HostCtx* c = nullptr;
   VP_TRY(get_ctx(2 * nslabs + 6, &c));
   cudaEvent_t ev_alloc = c->ev[0], ev_in0 = c->ev[1], ev_in = c->ev[2], ev_out = c->ev[3],
@@ -525,9 +522,9 @@ cudaError_t backward_pipeline(const IO& io, const float* angles, const Geom& g, 
   VP_TRY(cudaStreamWaitEvent(c->copy_out, ev_alloc, 0));
   VP_TRY(copy_angles(as, angles, g, c->copy_in));
   const size_t y0 = (size_t)a_split * ang_elems;
-  if (pieces) VP_TRY(io.angles_in(0, a_split, c->copy_in));
-  if (pieces) VP_TRY(cudaEventRecord(ev_in0, c->copy_in));
-  VP_TRY(io.angles_in(pieces ? a_split : 0, g.n_ang, c->copy_in));
+  if (a_split > 0) VP_TRY(io.angles_in(0, a_split, c->copy_in));
+  VP_TRY(cudaEventRecord(ev_in0, c->copy_in));
+  VP_TRY(io.angles_in(a_split, g.n_ang, c->copy_in));
   VP_TRY(cudaEventRecord(ev_in, c->copy_in));
   // the container slab by slab, in the order the results leave
   for (int k = 0; k < nslabs; ++k) {
@@ -548,7 +545,7 @@ cudaError_t backward_pipeline(const IO& io, const float* angles, const Geom& g, 
   if (a_split > 0) {
     Geom g0 = gs;
     g0.n_ang = a_split;
-    VP_TRY(cudaStreamWaitEvent(s, pieces ? ev_in0 : ev_in, 0));
+    VP_TRY(cudaStreamWaitEvent(s, ev_in0, 0));
     VP_TRY(launch_backward_z0_rows(yd, xd, ad, g0, 0, g.SY, s));
     *launches += launches_backward_z0(yd, xd, g0);
     g1.n_ang = g.n_ang - a_split;
