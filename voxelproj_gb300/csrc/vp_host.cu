@@ -621,17 +621,21 @@ cudaError_t z0_thin_host(bool forward, const float* in_host, float* out_host,
   }, s);
 }
 
-// Whether a pipeline pads its input's rows (z0_pads: whether a device call does).  The
-// pipelines run by pieces, which fill less of the GPU in the 256-height forward than
-// in the scalar form, and wait for the copies with few angles: A (512, 512, 203) and
-// 8 angles 1.97 ms on the input itself, 2.34 on padded rows; (128, 128, 257) and 30
-// 0.475 / 0.586, 120 angles 0.86 / 0.64; (64, 64, 257) and 120 0.326 / 0.354, 360
-// 0.63 / 0.41.
+// Whether a pipeline pads its input's rows (z0_pads: whether a device call does).  With
+// few angles a pipeline waits for the copies, and its pieces and groups of angles
+// fill less of the GPU on the float4 kernels than in the scalar form.  Calls on the
+// input itself / on padded rows, in ms: A (512, 512, 203) and 8 angles 1.97 / 2.34;
+// (128, 128, 257) and 30 0.475 / 0.586, 120 angles 0.86 / 0.64; (64, 64, 257) and 120
+// 0.326 / 0.354, 360 0.63 / 0.41; A^T (300, 300, 15) and 30 0.181 / 0.212, 90 0.351 / 0.299;
+// (64, 64, 33) and 60 0.083 / 0.088, 90 0.102 / 0.090.
 bool host_pads(int op, const Geom& g) {
   if (!z0_pads(op, g)) return false;
-  if (op != OP_FORWARD_Z0 || g.H <= 192) return true;
   const long long vox = (long long)g.SY * g.SX;
-  return g.n_ang >= (vox >= 192 * 192 ? 30 : vox >= 100 * 100 ? 100 : 240);
+  const int n = g.n_ang;
+  if (op == OP_FORWARD_Z0)
+    return g.H <= 192 || n >= (vox >= 192 * 192 ? 30 : vox >= 100 * 100 ? 100 : 240);
+  if (g.H <= 32) return n >= (vox >= 192 * 192 ? 90 : 120);
+  return n >= (vox >= 128 * 128 ? 30 : vox >= 64 * 64 ? 90 : 200);
 }
 
 // A second device buffer for a pipeline's input of rows x Hin floats at *dev, where
