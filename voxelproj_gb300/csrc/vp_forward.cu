@@ -162,6 +162,7 @@ struct Fp0Config {
   int band;       // banded form (vp_fp_band.cuh): runs per warp, 0 = candidate lists
   int staged;     // aligned neighbouring-angle forms (vp_fp_staged.cuh), 8 heights per
                   // lane only: 1 = staged by tensor copies, 2 = plain loads; 0 = none
+  int chunk_h = 128;  // height chunk of the candidate lists that a banded part replaces
 };
 
 // Variants: 1 = 4 bins per warp, 4 heights per lane, warps of a block on
@@ -310,15 +311,23 @@ Slab fp0_slab(const Geom& g, const Fp0Config& c, int k, int n) {
   return slab_of(k, c.cls, wy, wx, g.SY, g.SX);
 }
 
-// Lines per partial sum of the banded form (vp_fp_band.cuh): at most kBandLines, and no
-// more than a slab of 256-height chunks has.
-int fp0_band_lines(const Geom& g) {
-  Fp0Config c = fp0_config(g, false, 16);
-  c.R = 8;
+// Lines per partial sum of the banded form.  A bin's float32 error grows with the
+// number of lines that one accumulator runs over.  The candidate lists are launched
+// slab by slab (chunks of 128 or 256 heights; the banded form's slabs hold fewer
+// heights, so more lines) and split a run's lines over two warps in small grids; with
+// one sum over all lines the error against 64 bits was theirs times 1.5 (A (500, 512,
+// 32), 50 angles, precise: 2.25e-7 against 1.47e-7; with this 1.43e-7).  So: the
+// lists' slab width, and at most 64 and half of it where the lines are split, whose
+// partial sums gather in shared memory.  Unsplit they are added into y: sums of 64
+// lines took up to 8% longer there ((512, 512, 128), 78 angles 857 / 928 us).
+int fp0_band_lines(const Geom& g, const Fp0Config& c) {
+  Fp0Config lists = fp0_config(g, false, 16);
+  lists.R = c.chunk_h / 32;
   int wy = 0, wx = 0;
-  fp0_slab_widths(g, c, fp0_slabs(g, c), &wy, &wx);
+  fp0_slab_widths(g, lists, fp0_slabs(g, lists), &wy, &wx);
   const int w = wy > wx ? wy : wx;
-  return w < kBandLines ? w : kBandLines;
+  if (!c.split) return w;
+  return (w + 1) / 2 < 64 ? (w + 1) / 2 : 64;
 }
 
 // Rows of x take float4 loads; rows of y float4 stores.
@@ -486,7 +495,7 @@ cudaError_t launch_slab_aligned(const SlabLaunch& L, cudaStream_t stream, int* l
 cudaError_t launch_slab_config(const Fp0Config& c, const SlabLaunch& L, cudaStream_t s, int* n) {
   if (c.band)
     return launch_fp_band(BandLaunch{L.x, L.y, L.angles, L.g, L.slab, L.accumulate, L.a_lo, L.a_hi,
-                                     L.programmatic, L.vec_out, fp0_band_lines(L.g)},
+                                     L.programmatic, L.vec_out, fp0_band_lines(L.g, c)},
                           c.band, c.split, s, n);
   if (!L.vec_out && c.R != 1) {  // the default's forms (fp0_vec4)
     if (c.R == 8) return launch_slab<8, 4, true, 2, false, false, false>(L, s, n);
@@ -581,6 +590,13 @@ HeightParts fp0_parts(const Geom& g, bool vec4, int variant) {
   return p;
 }
 
+// The configuration of part i.
+Fp0Config fp0_part_config(const HeightParts& p, int i, bool vec4, int variant) {
+  Fp0Config c = fp0_config(p.g[i], vec4, variant);
+  if (p.n == 2 && p.h0[1] == 128) c.chunk_h = 256;  // fp0_parts_pay
+  return c;
+}
+
 cudaError_t launch_forward_z0(const float* x, float* y, const float* angles, const Geom& g,
                               cudaStream_t stream) {
   const bool vec4 = fp0_vec4(x, y, g);
@@ -588,7 +604,7 @@ cudaError_t launch_forward_z0(const float* x, float* y, const float* angles, con
   if (v == 0 && z0_forward_thin(g)) return launch_forward_thin(x, y, angles, g, 0, stream);
   const HeightParts hp = fp0_parts(g, vec4, v);
   for (int i = 0; i < hp.n; ++i) {
-    const Fp0Config c = fp0_config(hp.g[i], vec4, v);
+    const Fp0Config c = fp0_part_config(hp, i, vec4, v);
     const cudaError_t e = launch_fp_z0_config(x + hp.h0[i], y + hp.h0[i], angles, hp.g[i], c, 0,
                                               1 << 30, stream);
     if (e != cudaSuccess) return e;
@@ -618,7 +634,7 @@ int launches_forward_z0(const float* x, const float* y, const Geom& g) {
   const HeightParts hp = fp0_parts(g, vec4, v);
   int n = 0;
   for (int i = 0; i < hp.n; ++i) {
-    const Fp0Config c = fp0_config(hp.g[i], vec4, v);
+    const Fp0Config c = fp0_part_config(hp, i, vec4, v);
     const long long per =
         ((c.agroup && !c.band) || c.staged) ? (long long)kMaxGridYZ * FP0_WARPS : kMaxGridYZ;
     n += (int)(fp0_slabs(hp.g[i], c) * ceil_div(hp.g[i].n_ang, per));
@@ -677,8 +693,9 @@ cudaError_t launch_forward_z0_stream(const float* x, float* y, const float* angl
                                      cudaStream_t stream, int* launches) {
   const bool vec4 = fp0_vec4(x, y, g);
   const int v = kernel_variant(OP_FORWARD_Z0);
-  const Geom gm = fp0_parts(g, vec4, v).g[0];
-  Fp0Config c = fp0_config(gm, vec4, v);
+  const HeightParts hp = fp0_parts(g, vec4, v);
+  const Geom gm = hp.g[0];
+  Fp0Config c = fp0_part_config(hp, 0, vec4, v);
   c.cls = true;
   const SlabLaunch L{x, y, angles, gm, Slab{rows_lo, rows_hi, cols_lo, cols_hi, 0, g.SY},
                      accumulate, a_lo, a_hi, false, fp0_vec_out(y, gm)};
@@ -690,7 +707,7 @@ cudaError_t launch_forward_z0_rest(const float* x, float* y, const float* angles
   const bool vec4 = fp0_vec4(x, y, g);
   const HeightParts hp = fp0_parts(g, vec4, kernel_variant(OP_FORWARD_Z0));
   for (int i = 1; i < hp.n; ++i) {
-    const Fp0Config c = fp0_config(hp.g[i], vec4, kernel_variant(OP_FORWARD_Z0));
+    const Fp0Config c = fp0_part_config(hp, i, vec4, kernel_variant(OP_FORWARD_Z0));
     const cudaError_t e = launch_fp_z0_config(x + hp.h0[i], y + hp.h0[i], angles, hp.g[i], c, 0,
                                               1 << 30, stream, launches);
     if (e != cudaSuccess) return e;

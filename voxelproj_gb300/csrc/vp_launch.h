@@ -73,13 +73,6 @@ struct BandLaunch {
 cudaError_t launch_fp_band(const BandLaunch& L, int runs_per_warp, bool split,
                            cudaStream_t stream, int* launches);
 
-// Lines per partial sum of that form at most.  A bin's float32 error grows with the
-// number of lines that one accumulator runs over.  The candidate lists, launched slab
-// by slab and with a run's lines split over two warps in small grids, stay at about
-// this many; with one sum over all lines the error against 64 bits was theirs times
-// 1.5 (A (500, 512, 32), 50 angles, precise: 2.25e-7 against 1.47e-7; with this 1.43e-7).
-constexpr int kBandLines = 64;
-
 // The banded form's windows are placed with float coordinates, off by less
 // than its 0.05 voxels of margin up to here.
 inline bool fp0_band_ok(const Geom& g) {
