@@ -26,11 +26,16 @@ pytestmark = pytest.mark.gpu
     ("backward", 64, 64, 99, 60, 257, 1), ("backward", 130, 128, 33, 15, 130, 1),
     ("backward", 130, 128, 33, 16, 130, 3), ("backward", 130, 128, 31, 59, 130, 1),
     ("backward", 260, 256, 9, 29, 260, 1), ("backward", 260, 256, 9, 30, 260, 3),
-    ("backward", 30, 26, 257, 4, 30, 1),
+    ("backward", 30, 26, 257, 4, 30, 1), ("backward", 24, 24, 99, 59, 24, 1),
+    ("backward", 24, 24, 99, 60, 24, 3), ("backward", 96, 96, 203, 15, 96, 1),
+    ("backward", 96, 96, 203, 16, 96, 3), ("backward", 45, 45, 401, 59, 45, 1),
+    ("backward", 48, 48, 401, 60, 48, 3),
     ("forward", 24, 24, 131, 3, 24, 1), ("forward", 48, 48, 99, 1, 48, 2),
     ("forward", 24, 24, 203, 239, 24, 1), ("forward", 24, 24, 203, 240, 24, 2),
     ("forward", 70, 64, 203, 59, 70, 1), ("forward", 64, 64, 255, 60, 64, 2),
-    ("forward", 130, 128, 203, 29, 130, 1),
+    ("forward", 130, 128, 203, 29, 130, 1), ("forward", 36, 33, 203, 119, 36, 1),
+    ("forward", 36, 33, 203, 120, 36, 2), ("forward", 20, 100, 203, 120, 100, 1),
+    ("forward", 96, 96, 255, 59, 96, 1), ("forward", 40, 240, 255, 59, 240, 1),
 ])
 def test_copy_where_it_pays(op, SY, SX, H, n, PX, launches):
     ang = lin(n, -0.2, 3.3)

@@ -635,7 +635,8 @@ bool host_pads(int op, const Geom& g) {
   if (op == OP_FORWARD_Z0)
     return g.H <= 192 || n >= (vox >= 192 * 192 ? 30 : vox >= 100 * 100 ? 100 : 240);
   if (g.H <= 32) return n >= (vox >= 192 * 192 ? 90 : 120);
-  return n >= (vox >= 128 * 128 ? 30 : vox >= 64 * 64 ? 90 : 200);
+  if (vox >= 90 * 90) return n >= (vox >= 128 * 128 ? 30 : 60);
+  return n >= (vox >= 64 * 64 ? 90 : g.H <= 128 ? 120 : 200);
 }
 
 // A second device buffer for a pipeline's input of rows x Hin floats at *dev, where

@@ -133,16 +133,20 @@ cudaError_t pad_heights(const float* src, float* dst, long long rows, int Hs, in
 // angles or 48 x 48 voxels on.
 inline bool z0_pad_pays(int op, const Geom& g) {
   const long long vox = (long long)g.SY * g.SX;
+  const int least = g.SY < g.SX ? g.SY : g.SX;  // side
   const int n = g.n_ang;
   if (op == OP_FORWARD_Z0) {
     if (g.H <= 192) return g.H <= 128 || n >= 4 || vox >= 48 * 48;
     if (vox >= 320 * 320) return n >= (g.H <= 256 ? 1 : 8);
-    return n >= (vox >= 192 * 192 ? 16 : vox >= 128 * 128 ? 30 : vox >= 64 * 64 ? 60 : 240);
+    if (vox >= 128 * 128) return n >= (vox >= 192 * 192 ? 16 : 30);
+    if (vox >= 64 * 64) return n >= (g.H > 256 && least >= 90 ? 30 : 60);
+    return n >= (least >= 32 ? 120 : 240);
   }
   if (16ll * g.PX > vox) return false;  // (the sinogram is the copy)
-  if (vox < 128 * 128) return n >= (vox < 64 * 64 ? 120 : 60);
-  if (g.H > 32) return n >= 16;
-  return n >= (vox >= 256 * 256 ? 30 : 60);
+  if (vox >= 128 * 128) return n >= (g.H > 32 ? 16 : vox >= 256 * 256 ? 30 : 60);
+  if (vox >= 90 * 90 && g.H > 32) return n >= (g.H >= 200 ? 16 : 30);
+  if (vox >= 64 * 64 || g.H <= 128) return n >= 60;
+  return n >= (vox >= 45 * 45 && g.H >= 400 ? 60 : 120);
 }
 inline bool z0_pads(int op, const Geom& g) {
   return kernel_variant(op) == 0 &&
