@@ -23,6 +23,7 @@ pytestmark = pytest.mark.gpu
     (64, 64, 192, 264, 64, 2), (64, 64, 192, 268, 64, 1),    # a wave of 1064 blocks
     (64, 64, 400, 30, 64, 1), (64, 64, 448, 30, 64, 1),      # past 256 heights: no part of their own
     (64, 64, 300, 30, 64, 2),                                # a rest of at most 128: as ever
+    (500, 410, 132, 5, 500, 7), (500, 410, 132, 6, 500, 5),  # few angles, large: 7 slabs, 4 + 1
 ])
 def test_parts(SY, SX, H, n, PX, launches):
     ang = lin(n, -0.2, 3.3)

@@ -564,12 +564,14 @@ struct HeightParts {
 // per warp).  A in us, 256-height form / parts: 128 x 128 x 180 and 100 angles 190 /
 // 145, 400 angles 462 / 501; 256 x 256 x 180 and 30 angles 201 / 185, 200 angles
 // 889 / 977; 256 x 256 x 144 and 200 angles 866 / 689; 32 x 32 x 144 and 400
-// angles 47 / 49, 160 heights 47 / 53.  More than 256 heights stay in that form:
+// angles 47 / 49, 160 heights 47 / 53.  (498 x 498 x 136 and 3 angles, bound by HBM,
+// 159 / 171.)  More than 256 heights stay in that form:
 // 64 x 64 x 416 and 100 angles 95 against 128 in three parts, 512 x 512 x 416 and
 // 30 1387 against 1330.
 bool fp0_parts_pay(const Geom& g) {
   const long long blocks = (long long)ceil_div(g.PX, 4) * ceil_div(g.n_ang, FP0_WARPS);
   const long long vox = (long long)g.SY * g.SX;
+  if (g.H <= 160 && vox >= 448 * 448 && g.n_ang < 6) return false;
   return blocks <= (vox >= 64 * 64 ? 7 * 152 : 512) || (g.H <= 160 && vox >= 48 * 48);
 }
 
