@@ -190,9 +190,11 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
   const float* xs = x + h0 * st.xh;
   float(*tl)[LC][W] = tile[warp];
 
-  // each chunk of lines in a sum of its own: an accumulator that runs over a quarter of
-  // all lines had 1.2 times the error of the slabs' sums before it (A (500, 512, 4),
-  // 50 angles, precise)
+  // With 4 heights and more each chunk of lines has a sum of its own: an accumulator
+  // that runs over a quarter of all lines had 1.2 times the error of the candidate
+  // lists' slabs (A (500, 512, 4), 50 angles, precise).  Fewer heights replaced kernels
+  // with one sum over all lines (one slice 278.4 us, 279.8 with a sum per chunk).
+  constexpr bool kParts = RH >= 4;
   float acc[RH];
 #pragma unroll
   for (int h = 0; h < RH; ++h) acc[h] = 0.0f;
@@ -228,13 +230,13 @@ __global__ void __launch_bounds__(32 * THIN_WARPS)
     }
     __syncwarp();
     const ThinChunk c{i0, nl, m0, cent_major, cent_minor, sh_major, inv};
-    float part[RH];
+    float sum[RH];
 #pragma unroll
-    for (int h = 0; h < RH; ++h) part[h] = 0.0f;
-    if (minor_x) gather_lines<RH, LC, TRIG, true>(part, tl, c, fe, k, g.pcent);
-    else gather_lines<RH, LC, TRIG, false>(part, tl, c, fe, k, g.pcent);
+    for (int h = 0; h < RH; ++h) sum[h] = kParts ? 0.0f : acc[h];
+    if (minor_x) gather_lines<RH, LC, TRIG, true>(sum, tl, c, fe, k, g.pcent);
+    else gather_lines<RH, LC, TRIG, false>(sum, tl, c, fe, k, g.pcent);
 #pragma unroll
-    for (int h = 0; h < RH; ++h) acc[h] += part[h];
+    for (int h = 0; h < RH; ++h) acc[h] = kParts ? acc[h] + sum[h] : sum[h];
   }
 
   // the block's four sums
