@@ -31,7 +31,16 @@
  *   - work is enqueued on the caller's stream and never synchronises (the
  *     reference ran on the legacy default stream and synchronised through
  *     cudaFreeArray);
- *   - no per-call allocation or staging copy of the input.
+ *   - no per-call allocation or staging copy of the input, except
+ *       z_order 0 with input rows that are not whole 16-byte float4, where a
+ *       copy with padded rows pays for itself, and
+ *       z_order 2 without a caller's workspace (from 32 heights on; the
+ *       forward from 5):
+ *     both from stream-ordered pools of the library.  The padded copies' pool
+ *     (and that of z_order 2 below 32 heights) keeps at most 256 MB between
+ *     synchronisations.  Without memory for them kernels that need none run
+ *     (z_order 2 from 32 heights on: VP_ERR_CUDA), and so they do under stream
+ *     capture (z_order 2 from 32 heights on takes its scratch as a memory node).
  *
  * All pointers are device pointers on the current CUDA device.  `stream` is a
  * cudaStream_t (NULL = legacy default stream).

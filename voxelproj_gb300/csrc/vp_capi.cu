@@ -1,7 +1,8 @@
 // C ABI: argument validation, geometry setup and dispatch to the kernels.
 // The reference's host launchers (voxelproj/csrc/projectors.cu:34-299) also
-// copied the input into a cudaArray and bound a texture on every call; none
-// of that exists here, so a call is validation plus one kernel launch.
+// copied the input into a cudaArray and bound a texture on every call; here a
+// call is validation and kernel launches, with scratch from a stream-ordered
+// pool for z_order 2 and for rows that are not whole float4.
 #include <cuda_runtime.h>
 
 #include <atomic>

@@ -206,7 +206,7 @@ int fp0_sms() {
 // blocks fill less than a wave of 6 per SM, for sides above 64 up to 16 per SM, and
 // with one run per warp up to 12: split blocks are a quarter as long and level the
 // SMs better, at the price of one more weight table pass per warp where the lines
-// of a share fill no table.  A in us, unsplit / split: 32^3 and 128 angles (64 blocks)
+// of a share fill no table.  A in us, unsplit / split: 32^3 and 128 angles (128 blocks)
 // 16.5 / 8.3; 384 x 384 x 16 and 180 (540) 273 / 243; 128^3 and 125 (1000) 130 / 103,
 // 312 (2496) 241 / 231, 1000 (8000) 682 / 703; 256 x 256 x 16 and 150 (300) 148 / 106.
 // Volumes of at most 48 x 48 stay on the candidate lists (band 0) above 64 heights

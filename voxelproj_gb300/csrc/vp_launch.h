@@ -80,9 +80,9 @@ inline bool fp0_band_ok(const Geom& g) {
   return g.SY <= kMax && g.SX <= kMax && g.PX <= kMax;
 }
 // Its runs per warp: as many as leave a run the lanes for the heights (at most
-// 128).  A (213, 213, 40) and 492 angles 354 us with 2 runs, 293 with 3; 5 runs
-// at 17 to 24 heights gave nothing over 4 (256 x 256 x 20 170 us, 32 heights
-// with 4 163).
+// 128).  A (213, 213, 40) and 492 angles 564 us with 2 runs, 444 with 3, (300, 300, 40)
+// and 360 797 / 629; 5 runs at 17 to 24 heights gave nothing over 4 (256 x 256 x 20
+// and 180 angles 170 us, 32 heights with 4 163).
 inline int fp0_band_runs(int H) {
   return H <= 16 ? 8 : H <= 32 ? 4 : H <= 40 ? 3 : H <= 64 ? 2 : 1;
 }
