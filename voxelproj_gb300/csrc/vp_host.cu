@@ -165,6 +165,15 @@ bool is_device_pointer(const void* p) {
     if (e_ != cudaSuccess) return e_;        \
   } while (0)
 
+// `rows` rows of `width` bytes, `pitch` bytes apart on both sides.  A single row goes
+// as a 1-D copy: for pageable host memory a 2-D copy of one row touches the whole
+// pitch, past the end of the caller's array.
+cudaError_t copy_rows(void* dst, const void* src, size_t pitch, size_t width, size_t rows,
+                      cudaStream_t s) {
+  if (rows == 1) return cudaMemcpyAsync(dst, src, width, cudaMemcpyDefault, s);
+  return cudaMemcpy2DAsync(dst, pitch, src, pitch, width, rows, cudaMemcpyDefault, s);
+}
+
 // Angles on the device: the caller's pointer if it is device memory, else a
 // buffer (allocated here, filled by copy_angles on the copy stream).
 cudaError_t alloc_angles(const float* angles, const Geom& g, Buffers& buf, cudaMemPool_t pool,
@@ -263,10 +272,8 @@ struct FwdZ2IO {  // z_order 2 host arrays: strided blocks, transposed on the de
   size_t vox() const { return (size_t)g2.SY * g2.SX; }
   size_t bins() const { return (size_t)g2.n_ang * g2.PX; }
   cudaError_t rows_in(int lo, int hi, cudaStream_t copy) const {
-    VP_TRY(cudaMemcpy2DAsync(xs + (size_t)lo * g2.SX, vox() * sizeof(float),
-                             x_host + (size_t)lo * g2.SX, vox() * sizeof(float),
-                             (size_t)(hi - lo) * g2.SX * sizeof(float), g2.H, cudaMemcpyDefault,
-                             copy));
+    VP_TRY(copy_rows(xs + (size_t)lo * g2.SX, x_host + (size_t)lo * g2.SX, vox() * sizeof(float),
+                     (size_t)(hi - lo) * g2.SX * sizeof(float), g2.H, copy));
     *launches += 1;
     return z2_transpose_in_rows(xs, g2, ws, lo, hi, copy);
   }
@@ -278,10 +285,8 @@ struct FwdZ2IO {  // z_order 2 host arrays: strided blocks, transposed on the de
   cudaError_t send(int a0, int a1, cudaStream_t out, int* launches) const {
     VP_TRY(z2_transpose_out_angles(ys, g2, ws, a0, a1, g2.accumulate ? 1 : 0, out));
     *launches += 1;
-    return cudaMemcpy2DAsync(y_host + (size_t)a0 * g2.PX, bins() * sizeof(float),
-                             ys + (size_t)a0 * g2.PX, bins() * sizeof(float),
-                             (size_t)(a1 - a0) * g2.PX * sizeof(float), g2.H,
-                             cudaMemcpyDefault, out);
+    return copy_rows(y_host + (size_t)a0 * g2.PX, ys + (size_t)a0 * g2.PX, bins() * sizeof(float),
+                     (size_t)(a1 - a0) * g2.PX * sizeof(float), g2.H, out);
   }
 };
 
@@ -834,10 +839,9 @@ cudaError_t z2_backward_chunked(const float* y_host, float* x_host, const float*
             VP_TRY(z2_transpose_out_rows(dst, gj, ws[j & 1], lo, hi, g.accumulate ? 1 : 0,
                                          c->copy_out));
             *launches += 1;
-            VP_TRY(cudaMemcpy2DAsync(x_host + h0 * vox + (size_t)lo * g.SX, vox * sizeof(float),
-                                     dst + (size_t)lo * g.SX, vox * sizeof(float),
-                                     (size_t)(hi - lo) * g.SX * sizeof(float), hc,
-                                     cudaMemcpyDefault, c->copy_out));
+            VP_TRY(copy_rows(x_host + h0 * vox + (size_t)lo * g.SX, dst + (size_t)lo * g.SX,
+                             vox * sizeof(float), (size_t)(hi - lo) * g.SX * sizeof(float), hc,
+                             c->copy_out));
           }
           return cudaEventRecord(ev_done[j], c->copy_out);
         }
