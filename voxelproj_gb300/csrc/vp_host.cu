@@ -60,8 +60,11 @@ constexpr int kZ2AdjointSlabs = 8;    // row slabs of the z_order 2 adjoint's la
 // Blocks of one class launch that a row slab of an adjoint should hold at least
 // (5 resident blocks per SM: 1.5 waves).  Smaller slabs leave the GPU idle for
 // longer than they save in copies.  Host calls with and without the limit:
-// 256^3 and 360 angles 1.64 / 1.88 ms, (256, 256, 128) 0.93 / 1.31, 128 x 128 x
-// 100 and 200 0.30 / 0.65; 384 x 384 x 300 the same (4.01).
+// 256^3 and 360 angles 1.53 / 1.78 ms, (256, 256, 128) 0.93 / 1.31, 128 x 128 x
+// 100 and 200 0.30 / 0.65; 384 x 384 x 300 the same (4.01).  In z_order 0 half of it
+// above 128 heights with fewer than 256 angles, where the copies take more of the
+// call: (160, 160, 256) and 30 angles 0.29 / 0.31 ms with half / all of it (without
+// 0.31), (128, 128, 200) and 90 0.245 / 0.265 (0.41); 360 angles 1.59 / 1.53 at 256^3.
 constexpr long long kSlabBlocks = 1140;
 constexpr int kForwardAngleGroups = 4;  // groups of the forward's last slab
 // Forward angles sent home early: |phi| at most this many radians, and
@@ -489,11 +492,11 @@ struct BwdZ0IO {  // z_order 0 host arrays: contiguous row and angle blocks
   }
 };
 
-// Rows per adjoint slab: about SY / slabs, at least kSlabBlocks blocks of 4 x 4
+// Rows per adjoint slab: about SY / slabs, at least `blocks` blocks of 4 x 4
 // voxels by up to 256 heights, a multiple of step.
-int adjoint_slab_rows(const Geom& g, int slabs, int step) {
+int adjoint_slab_rows(const Geom& g, int slabs, int step, long long blocks) {
   const long long per_step = (long long)step * ((g.SX + 3) / 4) * ((g.H + 255) / 256);
-  const long long least = (4 * kSlabBlocks + per_step - 1) / per_step;
+  const long long least = (4 * blocks + per_step - 1) / per_step;
   long long steps = ((g.SY + slabs - 1) / slabs + step - 1) / step;
   if (steps < least) steps = least;
   return steps * step < g.SY ? (int)(steps * step) : g.SY;
@@ -508,7 +511,8 @@ cudaError_t backward_pipeline(const IO& io, const float* angles, const Geom& g, 
   const size_t ang_elems = (size_t)g.PX * g.Hy;
   const size_t x_elems = (size_t)g.SY * g.SX * g.Hx;
   const int step = backward_z0_row_step(yd, xd, g);
-  const int rows = step > 0 ? adjoint_slab_rows(g, kAdjointSlabs, step) : g.SY;
+  const long long blocks = g.H > 128 && g.n_ang < 256 ? kSlabBlocks / 2 : kSlabBlocks;
+  const int rows = step > 0 ? adjoint_slab_rows(g, kAdjointSlabs, step, blocks) : g.SY;
   const int nslabs = (g.SY + rows - 1) / rows;
   // the first sixth of the angles runs over the whole volume first, while
   // the rest of the sinogram arrives (at 512^3 with 192 angles, 12 slabs
@@ -779,7 +783,8 @@ cudaError_t z2_backward_chunked(const float* y_host, float* x_host, const float*
       gl.H = gl.Hx = gl.Hy = (int)(((size_t)gl.H + 3) / 4 * 4);
       const float* xtl = ws[(nchunks - 1) & 1];
       const int step = backward_z0_row_step(xtl + vox * gl.H, xtl, gl);
-      const int rows = step > 0 ? adjoint_slab_rows(gl, kZ2AdjointSlabs, step) : g.SY;
+      const int rows = step > 0 ? adjoint_slab_rows(gl, kZ2AdjointSlabs, step, kSlabBlocks)
+                                : g.SY;
       for (int q = 0; q < g.SY;) {
         q = q + rows < g.SY ? q + rows : g.SY;
         scut.push_back(q);
