@@ -39,7 +39,7 @@ def test_padding_starts_where_it_pays(S, H, line):
     assert below[0] == below[1] < _launches(S, H, line, check=S == 64)
 
 
-@pytest.mark.parametrize("S,H,line", [(64, 9, 120), (192, 15, 90), (128, 33, 30), (64, 33, 90), (96, 99, 60), (30, 99, 120), (30, 203, 200)])
+@pytest.mark.parametrize("S,H,line", [(64, 9, 120), (192, 15, 90), (128, 33, 45), (128, 99, 30), (64, 33, 90), (96, 99, 60), (30, 99, 120), (30, 203, 200)])
 def test_adjoint_padding_starts_where_it_pays(S, H, line):
     below = [_launches(S, H, n, True, forward=False) for n in (line // 2, line - 1)]
     assert below[0] == below[1] < _launches(S, H, line, True, forward=False)

@@ -636,7 +636,8 @@ cudaError_t z0_thin_host(bool forward, const float* in_host, float* out_host,
 // input itself / on padded rows, in ms: A (512, 512, 203) and 8 angles 1.97 / 2.34;
 // (128, 128, 257) and 30 0.475 / 0.586, 120 angles 0.86 / 0.64; (64, 64, 257) and 120
 // 0.326 / 0.354, 360 0.63 / 0.41; A^T (300, 300, 15) and 30 0.181 / 0.212, 90 0.351 / 0.299;
-// (64, 64, 33) and 60 0.083 / 0.088, 90 0.102 / 0.090.
+// (140, 140, 35), 203 bins and 30 0.113 / 0.128; (64, 64, 33) and 60 0.083 / 0.088,
+// 90 0.102 / 0.090.
 bool host_pads(int op, const Geom& g) {
   if (!z0_pads(op, g)) return false;
   const long long vox = (long long)g.SY * g.SX;
@@ -644,7 +645,7 @@ bool host_pads(int op, const Geom& g) {
   if (op == OP_FORWARD_Z0)
     return g.H <= 192 || n >= (vox >= 192 * 192 ? 30 : vox >= 100 * 100 ? 100 : 240);
   if (g.H <= 32) return n >= (vox >= 192 * 192 ? 90 : 120);
-  if (vox >= 90 * 90) return n >= (vox >= 128 * 128 ? 30 : 60);
+  if (vox >= 90 * 90) return n >= (vox < 128 * 128 ? 60 : g.H < 64 ? 45 : 30);
   return n >= (vox >= 64 * 64 ? 90 : g.H <= 128 ? 120 : 200);
 }
 
